@@ -821,6 +821,7 @@ int qx_ens_set_mixed(qx_ens_t* h, int mixed) {
             if (e.exec) cudaGraphExecDestroy(e.exec);
             e.exec = nullptr;
             e.mixed = mixed;
+            for (auto& g : e.groups) g->set_planes(mixed == 0);
         }
     });
 }

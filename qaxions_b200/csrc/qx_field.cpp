@@ -13,6 +13,7 @@
 #include <string>
 
 #include "qx_misc.hpp"
+#include "qx_plane.hpp"
 #include "qx_philox.h"
 
 namespace qx {
@@ -491,7 +492,23 @@ class FieldT final : public Field {
         s.phase_fac = -0.5 * dt * dk() * dk();
         s.scale = 1.0 / (double)g_.S1;
         s.axy = ensure_axy(dt);
-        Ops<R>::la_pass(g_.N, s, OP_DRIFT, tune_, st_);
+        last_axis(s, OP_DRIFT);
+    }
+    // the drift and Poisson passes along the last axis: the direct-load column
+    // kernels where the grid has them, else the tile ring
+    bool col_on() const { return tune_.tma && tune_.plan == 0 && planes_ && Plane<R>::col(g_.N, g_.dim); }
+    void last_axis(const typename Ops<R>::SP& s, int op) {
+        if (col_on()) Plane<R>::col_pass(g_.N, s, op, st_);
+        else Ops<R>::la_pass(g_.N, s, op, tune_, st_);
+    }
+    // 3D boxes whose z planes fit an SM's shared memory: the x and y transforms of
+    // a plane (and the pointwise work between them) in one launch; between the
+    // launches of the merged loop psi is then transformed along x and y (psi^_xy)
+    // instead of along x only
+    bool planes_on() const { return g_.dim == 3 && Plane<R>::xy(g_.N) && col_on() && !chain_on(); }
+    void set_planes(bool on) override {
+        if (on != planes_) invalidate_graph();
+        planes_ = on;
     }
     // psi^_x -> y forward, z drift, y inverse: one slab-ordered kernel (FP32
     // 3D, tune_.chain) or three passes
@@ -506,15 +523,43 @@ class FieldT final : public Field {
             Ops<R>::drift_chain(g_.N, s, tune_.chain, chain_.as<unsigned>(), tune_, st_);
             return;
         }
+        if (planes_on()) {
+            la_drift(dt);
+            return;
+        }
         y_fwd(psi(), g_.N);
         la_drift(dt);
         y_inv(psi(), g_.N);
+    }
+    // psi^ as yz_drift leaves it -> psi; with r2c also the density's half
+    // spectrum, transformed along all axes but the last
+    void psi_inverse(const typename Ops<R>::XP& a, bool r2c) {
+        if (planes_on()) {
+            Plane<R>::inv(g_.N, a, r2c, st_);
+            return;
+        }
+        Ops<R>::x_inv(g_.N, a, r2c, tune_, st_);
+        if (r2c) y_fwd(vh(), g_.N / 2);
+    }
+    // psi (kicked by a.Vin first if kick) -> psi^ as yz_drift takes it
+    void psi_forward(const typename Ops<R>::XP& a, bool kick) {
+        if (planes_on()) Plane<R>::fwd(g_.N, a, kick, st_);
+        else Ops<R>::x_fwd(g_.N, a, kick, tune_, st_);
+    }
+    // the half spectrum after the last-axis Poisson pass -> V, then as the C2R flags say
+    void potential_c2r(const typename Ops<R>::XP& a, int flags) {
+        if (planes_on()) {
+            Plane<R>::c2r(g_.N, a, flags, st_);
+            return;
+        }
+        y_inv(vh(), g_.N / 2);
+        Ops<R>::x_c2r(g_.N, a, flags, tune_, st_);
     }
     void la_poisson() {
         auto s = sp(vh(), g_.N / 2);
         s.pois_c = pois_c();
         s.pois_g0 = pois_g0();
-        Ops<R>::la_pass(g_.N, s, OP_POISSON, tune_, st_);
+        last_axis(s, OP_POISSON);
     }
     // density source -> half spectrum, transformed along all axes but the
     // last (ready for the fused last-axis Poisson pass)
@@ -524,6 +569,10 @@ class FieldT final : public Field {
         a.vh = vh();
         a.pref = pref_eff();
         a.rho_mean = cfg_.rho_mean;
+        if (planes_on()) {
+            Plane<R>::r2c(g_.N, a, st_);
+            return;
+        }
         Ops<R>::x_r2c(g_.N, a, false, tune_, st_);
         y_fwd(vh(), g_.N / 2);
     }
@@ -535,9 +584,9 @@ class FieldT final : public Field {
         auto a = xp();
         a.in = psi();
         a.out = psi();
-        Ops<R>::x_fwd(g_.N, a, false, tune_, st_);
+        psi_forward(a, false);
         yz_drift(dt);
-        Ops<R>::x_inv(g_.N, a, false, tune_, st_);
+        psi_inverse(a, false);
         v_current_ = false;
     }
 
@@ -549,11 +598,10 @@ class FieldT final : public Field {
     void updatePotential() override {  // src/field.cxx:294-346
         density_r2c_partial();
         la_poisson();
-        y_inv(vh(), g_.N / 2);
         auto a = xp();
         a.vh = vh();
         a.Vout = V();
-        Ops<R>::x_c2r(g_.N, a, C2R_WRITE_V, tune_, st_);
+        potential_c2r(a, C2R_WRITE_V);
         v_current_ = true;
         vmax_ = reduce(RED_VABS)[1];
     }
@@ -570,14 +618,13 @@ class FieldT final : public Field {
     void prologue() {
         density_r2c_partial();
         la_poisson();
-        y_inv(vh(), g_.N / 2);
         auto a = xp();
         a.in = psi();
         a.out = psi();
         a.vh = vh();
         a.Vout = V();
         a.dt = 0.5 * ds_;
-        Ops<R>::x_c2r(g_.N, a, C2R_KICK | C2R_FWD, tune_, st_);
+        potential_c2r(a, C2R_KICK | C2R_FWD);
     }
 
     // fused merged leapfrog (src/main.cxx:64-85)
@@ -653,17 +700,10 @@ class FieldT final : public Field {
         a.Vout = V();
         a.pref = pref;
         a.rho_mean = cfg_.rho_mean;
-        Ops<R>::x_inv(g_.N, a, true, tune_, st_);
-        y_fwd(vh(), g_.N / 2);
+        psi_inverse(a, true);
         la_poisson();
-        y_inv(vh(), g_.N / 2);
-        if (last) {
-            a.dt = 0.5 * dt_kick;
-            Ops<R>::x_c2r(g_.N, a, C2R_WRITE_V | C2R_KICK | C2R_WRITE_PSI, tune_, st_);
-        } else {
-            a.dt = dt_kick;
-            Ops<R>::x_c2r(g_.N, a, C2R_KICK | C2R_FWD, tune_, st_);
-        }
+        a.dt = last ? 0.5 * dt_kick : dt_kick;
+        potential_c2r(a, last ? C2R_WRITE_V | C2R_KICK | C2R_WRITE_PSI : C2R_KICK | C2R_FWD);
     }
 
     // ---- measured time loop (src/main.cxx:60-85, src/meas.cxx:13-63) ----
@@ -679,11 +719,9 @@ class FieldT final : public Field {
         a.Vout = V();
         a.pref = pref;
         a.rho_mean = cfg_.rho_mean;
-        Ops<R>::x_inv(g_.N, a, true, tune_, st_);
-        y_fwd(vh(), g_.N / 2);
+        psi_inverse(a, true);
         la_poisson();
-        y_inv(vh(), g_.N / 2);
-        Ops<R>::x_c2r(g_.N, a, C2R_WRITE_V, tune_, st_);
+        potential_c2r(a, C2R_WRITE_V);
     }
 
     void measure(unsigned mask, int number, const char* dir, MeasRecord* rec) override {
@@ -804,7 +842,7 @@ class FieldT final : public Field {
             a.Vin = V();
             if (!last) {  // full_kick, then x forward for the next drift
                 a.dt = ds_;
-                Ops<R>::x_fwd(g_.N, a, true, tune_, st_);
+                psi_forward(a, true);
             } else {      // the final half_kick (src/main.cxx:82)
                 Misc<R>::kick(psi(), V(), 0.5 * ds_, g_.S, st_);
             }
@@ -1357,35 +1395,39 @@ class FieldT final : public Field {
     // per-pass device time of the loop body, averaged over nsteps bodies
     void profile_step(int nsteps, std::vector<std::pair<std::string, double>>& out) override {
         const bool d3 = g_.dim == 3;
-        const bool chain = chain_on();
+        const bool chain = chain_on(), planes = planes_on();
         std::vector<std::string> names;
-        if (chain) {
+        if (planes) {
+            names = {"z_drift(psi)", "yx_inv_r2c_y(psi->rho^)", "z_poisson(rho^)", "yx_c2r_kick_fwd_y"};
+        } else if (chain) {
             names.push_back("yzy_drift_chain(psi)");
         } else {
             if (d3) names.push_back("y_fwd(psi)");
             names.push_back(d3 ? "z_drift(psi)" : "y_drift(psi)");
             if (d3) names.push_back("y_inv(psi)");
         }
-        names.push_back("x_inv_r2c(psi->rho^)");
-        if (d3) names.push_back("y_fwd(rho^)");
-        names.push_back(d3 ? "z_poisson(rho^)" : "y_poisson(rho^)");
-        if (d3) names.push_back("y_inv(rho^)");
-        names.push_back("x_c2r_kick_fwd");
+        if (!planes) {
+            names.push_back("x_inv_r2c(psi->rho^)");
+            if (d3) names.push_back("y_fwd(rho^)");
+            names.push_back(d3 ? "z_poisson(rho^)" : "y_poisson(rho^)");
+            if (d3) names.push_back("y_inv(rho^)");
+            names.push_back("x_c2r_kick_fwd");
+        }
         const size_t np = names.size();
         std::vector<cudaEvent_t> ev(np + 1);
         for (auto& e : ev) QX_CUDA(cudaEventCreate(&e));
         std::vector<double> acc(np, 0.0);
-        {  // the loop body expects the x-transformed state
+        {  // the loop body expects the transformed state
             auto a = xp();
             a.in = psi();
             a.out = psi();
-            Ops<R>::x_fwd(g_.N, a, false, tune_, st_);
+            psi_forward(a, false);
         }
         for (int it = 0; it < nsteps; ++it) {
             size_t k = 0;
             QX_CUDA(cudaEventRecord(ev[0], st_));
             auto mark = [&]() { QX_CUDA(cudaEventRecord(ev[++k], st_)); };
-            if (chain) {
+            if (chain || planes) {
                 yz_drift(ds_); mark();
             } else {
                 if (d3) { y_fwd(psi(), g_.N); mark(); }
@@ -1395,11 +1437,17 @@ class FieldT final : public Field {
             auto a = xp();
             a.in = psi(); a.out = psi(); a.vh = vh(); a.Vout = V();
             a.pref = pref_eff(); a.rho_mean = cfg_.rho_mean; a.dt = ds_;
-            Ops<R>::x_inv(g_.N, a, true, tune_, st_); mark();
-            if (d3) { y_fwd(vh(), g_.N / 2); mark(); }
-            la_poisson(); mark();
-            if (d3) { y_inv(vh(), g_.N / 2); mark(); }
-            Ops<R>::x_c2r(g_.N, a, C2R_KICK | C2R_FWD, tune_, st_); mark();
+            if (planes) {
+                psi_inverse(a, true); mark();
+                la_poisson(); mark();
+                potential_c2r(a, C2R_KICK | C2R_FWD); mark();
+            } else {
+                Ops<R>::x_inv(g_.N, a, true, tune_, st_); mark();
+                if (d3) { y_fwd(vh(), g_.N / 2); mark(); }
+                la_poisson(); mark();
+                if (d3) { y_inv(vh(), g_.N / 2); mark(); }
+                Ops<R>::x_c2r(g_.N, a, C2R_KICK | C2R_FWD, tune_, st_); mark();
+            }
             QX_CUDA(cudaEventSynchronize(ev[np]));
             for (size_t j = 0; j < np; ++j) {
                 float ms = 0.f;
@@ -1416,13 +1464,13 @@ class FieldT final : public Field {
     }
 
     void restore_after_profile() {
-        // psi holds the x-transformed state after a full kick; undo the x
-        // transform (1/N) so the field is back in real space.
+        // psi holds the transformed state after a full kick; undo the x (1/N) or
+        // x and y (1/N^2) transforms so the field is back in real space.
         auto a = xp();
         a.in = psi();
         a.out = psi();
-        a.scale = 1.0 / (double)g_.N;
-        Ops<R>::x_inv(g_.N, a, false, tune_, st_);
+        a.scale = planes_on() ? 1.0 / ((double)g_.N * g_.N) : 1.0 / (double)g_.N;
+        psi_inverse(a, false);
         QX_CUDA(cudaStreamSynchronize(st_));
         v_current_ = false;
         vmax_stale_ = true;
@@ -1459,6 +1507,7 @@ class FieldT final : public Field {
     DevBuf mpsi_, mvh_, kin_, specP_, specC_, stage_;
     std::map<long, std::unique_ptr<DevBuf>> bintab_;
     std::unique_ptr<B200FFTBackend<R>> fft_;
+    bool planes_ = true;  // plane-resident and direct-load passes allowed (set_planes)
     bool v_current_ = false;
     bool vmax_stale_ = true;
     bool graph_enabled_ = true;

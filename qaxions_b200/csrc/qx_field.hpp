@@ -170,6 +170,10 @@ class Field {
     // the device arrays, tables and loop-body constants one pass launch over
     // several fields of different sizes needs (3D; after prepare_replay)
     virtual void mix_desc(MixDesc& d) = 0;
+    // allow (default) or forbid the plane-resident passes, whose loop body takes
+    // psi transformed along x and y: a caller that runs the body itself on the
+    // x-transformed state (mix_desc) forbids them before step_begin
+    virtual void set_planes(bool on) = 0;
     // measure() (src/meas.cxx:13-63) without overwriting V (unless the mask
     // has MEAS_CLOBBER_V); files go to `dir` when it is not null
     virtual void measure(unsigned mask, int number, const char* dir, MeasRecord* rec) = 0;

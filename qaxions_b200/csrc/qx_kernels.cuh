@@ -27,6 +27,12 @@
 
 namespace qx {
 
+// programmatic dependent launch: let the next kernel of the stream start its
+// prologue; wait until every earlier kernel has finished and its writes are
+// visible (both no-ops for a kernel launched without the attribute)
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---------------------------------------------------------------------------
 // shared-memory accessors
 // ---------------------------------------------------------------------------

@@ -9,17 +9,12 @@
 #include <cudaTypedefs.h>
 
 #include "qx_kernels.cuh"
+#include "qx_launch.cuh"
 #include "qx_ops.hpp"
 #include "qx_tma.cuh"
 #include "qx_yzy.cuh"
 
 namespace qx {
-
-#define QX_LAUNCH_CHECK()                                                                 \
-    do {                                                                                  \
-        cudaError_t e_ = cudaGetLastError();                                              \
-        if (e_ != cudaSuccess) throw std::runtime_error(std::string("kernel launch: ") + cudaGetErrorString(e_)); \
-    } while (0)
 
 // Dispatch a template functor over the supported N.
 #define QX_FOR_N(N, ...)                      \
@@ -35,29 +30,6 @@ namespace qx {
         case 512: { constexpr int NN = 512; __VA_ARGS__; break; } \
         default: throw std::invalid_argument("unsupported grid size N=" + std::to_string(N)); \
     }
-
-template <typename K>
-static void set_smem(K kernel, size_t bytes) {
-    if (bytes > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-        if (e != cudaSuccess) throw std::runtime_error(std::string("smem attribute: ") + cudaGetErrorString(e));
-    }
-}
-
-template <typename R> static XArgs<R> to_x(const typename Ops<R>::XP& a) {
-    XArgs<R> x;
-    x.in = a.in; x.out = a.out; x.vh = a.vh; x.Vin = a.Vin; x.Vout = a.Vout;
-    x.twN = a.twN; x.twM = a.twM; x.twN_lo = a.twN_lo; x.twM_lo = a.twM_lo; x.twNn = a.twNn;
-    x.rows = a.rows; x.dt = a.dt; x.pref = a.pref;
-    x.rho_mean = a.rho_mean; x.scale = a.scale;
-    return x;
-}
-template <typename R> static SArgs<R> to_s(const typename Ops<R>::SP& a) {
-    SArgs<R> s;
-    s.a = a.a; s.tw = a.tw; s.tw_lo = a.tw_lo; s.X = a.X; s.dim = a.dim; s.N = a.N; s.phase_fac = a.phase_fac;
-    s.scale = a.scale; s.pois_c = a.pois_c; s.pois_g0 = a.pois_g0; s.partial = a.partial;
-    return s;
-}
 
 template <typename R>
 void Ops<R>::stage_twiddles(const C* nat, int L, C* out) {
