@@ -447,7 +447,9 @@ class Field:
         16-column swizzled tiles for the wave-function passes (1 / True), for
         every strided pass (2), or 8-column tiles everywhere (0 / False); at
         N = 512, 3 / 4 split each pencil pair over two warps in the drift pass /
-        in every wave-function pass (bit for bit 1)."""
+        in every wave-function pass (bit for bit 1).  FP64 at N = 512: any
+        non-zero value runs the wave-function and Poisson passes with one or
+        two warps per pencil."""
         self._c("qx_set_pencil_warp", int(on))
 
     def set_row_stage(self, on):

@@ -438,10 +438,11 @@ class FieldT final : public Field {
         QX_CUDA(cudaMemsetAsync(V_.p, 0, V_.bytes, st_));
         QX_CUDA(cudaMemsetAsync(vh_.p, 0, vh_.bytes, st_));
         fft_ = std::make_unique<B200FFTBackend<R>>(g_, tw_, &tune_, st_, err_);
-        // measured default: at 512^3 FP32 the wave-function passes run faster with
-        // one warp per pencil pair (the drift pass with two warps per pair), the
-        // half-spectrum passes with the 8-column tiles
-        if (sizeof(R) == 4 && cfg.dim == 3 && cfg.N == 512) tune_.wp = 3;
+        // measured default at 512^3: FP32, the wave-function passes with one warp per
+        // pencil pair (the drift pass with two warps per pair), the half-spectrum
+        // passes with the 8-column tiles; FP64, one warp per pencil in the
+        // wave-function passes and two in the Poisson pass (launch_tma_tx)
+        if (cfg.dim == 3 && cfg.N == 512) tune_.wp = sizeof(R) == 4 ? 3 : 1;
         consult_tune_cache();
         // drift chain: phase counters (as many as 8-column slabs need)
         chain_n_ = Ops<R>::chain_slabs(g_.N, g_.dim, g_.B, 1);
@@ -1323,14 +1324,15 @@ class FieldT final : public Field {
         // (wp 1, the half-spectrum passes on the default tiles) or all (wp 2); at
         // N = 512 also two warps per pair in the drift pass (3) or in every
         // wave-function pass (4)
-        if (sizeof(R) == 4 && (g_.N == 256 || g_.N == 512))
+        if ((sizeof(R) == 4 && g_.N == 256) || g_.N == 512)
             for (int wp : {1, 2, 3, 4}) {
                 if (wp > 2 && g_.N != 512) continue;
+                if (wp > 1 && sizeof(R) == 8) continue;  // one form in FP64
                 for (int nb : {0, 2})
                     for (int xr : {0, 4}) {
                         Tune t;
                         t.wp = wp;
-                        t.pw = 2;
+                        t.pw = pws[0];
                         t.nbuf = nb;
                         t.x_rows = xr;
                         t.tma = 1;

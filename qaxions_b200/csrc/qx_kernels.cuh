@@ -691,8 +691,18 @@ template <typename R> __device__ __forceinline__ R pois_mult(long M2, const SArg
 template <> __device__ __forceinline__ float pois_mult<float>(long M2, const SArgs<float>& s) {
     return M2 == 0 ? (float)s.pois_g0 : (float)s.pois_c * __frcp_rn((float)M2);
 }
+// pois_c / M2 in FP64 without the general division's range checks: |n|^2 is an
+// integer below 2^24, exact in FP32, so its FP32 reciprocal takes two
+// Newton-Raphson steps to full precision, and the quotient one residual
+// correction (Markstein's division scheme), which rounds it as the division does
 template <> __device__ __forceinline__ double pois_mult<double>(long M2, const SArgs<double>& s) {
-    return M2 == 0 ? s.pois_g0 : s.pois_c / (double)M2;
+    if (M2 == 0) return s.pois_g0;
+    const double m = (double)(int)M2;
+    double x = (double)__frcp_rn((float)(int)M2);
+    x = fma(x, fma(-m, x, 1.0), x);
+    x = fma(x, fma(-m, x, 1.0), x);
+    const double q = s.pois_c * x;
+    return fma(fma(-q, m, s.pois_c), x, q);
 }
 
 // Last-axis pass.  3D: pencils along z of [N][N][X]; blockIdx = (x tile,

@@ -323,15 +323,15 @@ static long launch_tma_e(const typename Ops<R>::SP& a, int NZ, int outer, int pe
     return grid;
 }
 
-// Warp-per-pencil-pair pass (k_pencil_wp): FP32, N = 256 / 512, paired
-// pencils, 16-column swizzled tiles, a 3-deep ring, one block per SM of 8 warps
-// (WPP = 1) or 16 warps, two per pencil pair (WPP = 2).
+// Warp-per-pencil pass (k_pencil_wp): N = 256 / 512, 128-byte swizzled rows of 8
+// pencil units (FP32 pencil pairs, FP64 single pencils), a 3-deep ring, one
+// block per SM of 8 warps (WPP = 1) or 16 warps, two per unit (WPP = 2).
 template <int NN, typename R, int OP, bool DF, int WPP = 1>
 static long launch_wp(const typename Ops<R>::SP& a, int NZ, int outer, int pencil_dim, int la3d, int col0_ext,
                       cudaStream_t st) {
-    if constexpr (sizeof(R) == 4 && wp_supported(NN)) {
-        constexpr int TX = kWpTX;
-        if (a.X % TX) throw std::logic_error("warp-pencil pass: columns not a multiple of 16");
+    if constexpr (wp_supported(NN)) {
+        constexpr int TX = wp_tx<R>();
+        if (a.X % TX) throw std::logic_error("warp-pencil pass: columns not a multiple of the tile");
         TArgs<R> s;
         s.tw = a.tw;
         s.tw_lo = a.tw_lo;
@@ -356,7 +356,7 @@ static long launch_wp(const typename Ops<R>::SP& a, int NZ, int outer, int penci
         s.partial = a.partial;
         s.err = a.err;
         const CUtensorMap tm = make_tmap<R>(a.a, a.X, NN, NZ, TX, s.box, pencil_dim, true);
-        auto kern = k_pencil_wp<NN, OP, DF, 0, WPP>;
+        auto kern = k_pencil_wp<NN, R, OP, DF, 0, WPP>;
         const size_t smem = tma_smem_bytes<R>(NN, TX, s.nbuf, OP, true);
         set_smem(kern, smem);
         long grid = (long)sm_count();
@@ -392,6 +392,19 @@ static long launch_tma_tx(const typename Ops<R>::SP& a, int NZ, int outer, int p
                         return launch_wp<NN, R, OP, DF, 2>(a, NZ, outer, pencil_dim, la3d, col0_ext, st);
                 }
                 return launch_wp<NN, R, OP, DF>(a, NZ, outer, pencil_dim, la3d, col0_ext, st);
+            }
+        }
+        if constexpr (sizeof(R) == 8 && NN == 512) {
+            // FP64 512: the psi passes with one warp per pencil, the Poisson pass with two
+            // (128 registers a thread; its second array of values, the multipliers, costs
+            // one warp per pencil 255); y passes of the half spectrum stay on the plain tiles
+            // (HBM-bound in both).  Measured, us, plain tiles -> this: z drift 2173 -> 1177
+            // (two warps 1428), z Poisson 1144 -> 725 (one warp 851), y forward / inverse
+            // 783 / 771 -> 752 / 742; the step 8.70 -> 7.10 ms.  At 256 the plain tiles are faster throughout (y forward
+            // 100 against 122), so it is not compiled there.
+            if (a.plan == 0 && tu.wp != 0) {
+                if constexpr (OP == OP_POISSON) return launch_wp<NN, R, OP, DF, 2>(a, NZ, outer, pencil_dim, la3d, col0_ext, st);
+                else if (a.X == NN) return launch_wp<NN, R, OP, DF>(a, NZ, outer, pencil_dim, la3d, col0_ext, st);
             }
         }
         if constexpr (strided_plan1<NN>()) {

@@ -451,12 +451,14 @@ __global__ void __launch_bounds__((tma_block_threads<N, R, PW, TXF>()), (tma_blo
 }
 
 // ---------------------------------------------------------------------------
-// Warp-per-pencil-pair strided pass (FP32, N = 256 or 512).
+// Warp-per-pencil-pair strided pass (FP32 N = 256 or 512, FP64 N = 512).
 //
 // Tiles of 16 columns x N positions (128-byte rows, TMA 128-byte swizzle: the
 // 16-byte pencil pair q of row r sits in chunk q ^ (r & 7)) stream through a
 // 3-deep ring; one block of 8 warps per SM; warp w transforms the pencil pair
 // of columns x0 + 2w, x0 + 2w + 1 with E = N/32 values of each pencil per lane.
+// In FP64 a tile has 8 columns and warp w's unit is the single pencil of column
+// x0 + w: the same 16-byte units, slots and exchanges.
 // A pencil pair lives in its warp's own 16-byte slots of the tile, so the FFT
 // stage exchanges need only __syncwarp: the block synchronises once per tile,
 // before the tensor store.  The exchanges address element p at row
@@ -489,8 +491,10 @@ template <typename P, int WPP = 1> struct WarpXAcc {
     __device__ __forceinline__ void sync() const { pair_sync<WPP>(c); }
 };
 
-constexpr int kWpTX = 16;        // tile columns
-constexpr int kWpThreads = 256;  // 8 warps, one pencil pair each
+// tile columns: 8 pencil units of 16 bytes (a pair of FP32 pencils or one FP64
+// pencil) per 128-byte row
+template <typename R> __host__ __device__ constexpr int wp_tx() { return sizeof(R) == 4 ? 16 : 8; }
+constexpr int kWpThreads = 256;  // 8 warps, one pencil unit each
 
 __host__ __device__ constexpr bool wp_supported(int N) { return N == 256 || N == 512; }
 
@@ -502,19 +506,19 @@ __host__ __device__ constexpr bool wp_supported(int N) { return N == 256 || N ==
 // and radix-8 stages every exchange stays conflict-free (each 8-lane phase of
 // an access meets 8 distinct rows mod 8 after sigma).
 // blockDim = (32 WPP, 8): thread t = threadIdx.x of pencil pair c = threadIdx.y
-template <int N, int OP, bool DF, int PLAN = 0, int WPP = 1>
-__global__ void __launch_bounds__(kWpThreads * WPP, 1) k_pencil_wp(const __grid_constant__ CUtensorMap tm, TArgs<float> s) {
-    using R = float;
-    using C = float2;
-    using P = CPair<C>;
+template <int N, typename R, int OP, bool DF, int PLAN = 0, int WPP = 1>
+__global__ void __launch_bounds__(kWpThreads * WPP, 1) k_pencil_wp(const __grid_constant__ CUtensorMap tm, TArgs<R> s) {
+    using C = cx_t<R>;
+    constexpr int PW = sizeof(R) == 4 ? 2 : 1;  // pencils per unit
+    using P = pencil_val_t<PW, C>;
+    static_assert(sizeof(P) == 16, "a pencil unit is 16 bytes");
     static_assert(wp_supported(N), "warp-per-pencil passes are compiled for N = 256, 512");
-    static_assert(WPP == 1 || (WPP == 2 && N == 512 && (OP == OP_FWD || OP == OP_INV || OP == OP_DRIFT)),
-                  "two warps per pencil pair: N = 512 wave-function passes only");
+    static_assert(WPP == 1 || (WPP == 2 && N == 512), "two warps per pencil unit: N = 512 only");
     constexpr int NL = qx_with_plan(N, PLAN);
     constexpr int TPP = 32 * WPP;
     constexpr int E = N / TPP;
     static_assert(E % qx_lcm_radices(NL) == 0, "values per thread must hold whole butterflies");
-    constexpr int TX = kWpTX;
+    constexpr int TX = wp_tx<R>();
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t mbar[8];
     __shared__ int s_abort;
@@ -582,7 +586,7 @@ __global__ void __launch_bounds__(kWpThreads * WPP, 1) k_pencil_wp(const __grid_
         C* tile = bufs + b * tile_elems;
         const int x0 = (int)(id % s.tiles_x) * TX;
         const int o = (int)(id / s.tiles_x);
-        const int xb = x0 + 2 * c;
+        const int xb = x0 + PW * c;
         SwzRowAcc<P, WPP> io{reinterpret_cast<P*>(tile), c};
         WarpXAcc<P, WPP> acc{reinterpret_cast<P*>(tile), c};
         const long id_next = id + gridDim.x;
@@ -610,7 +614,7 @@ __global__ void __launch_bounds__(kWpThreads * WPP, 1) k_pencil_wp(const __grid_
         bool store = true;
         if constexpr (OP == OP_KIN) {
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
+            for (int h = 0; h < PW; ++h) {
                 const long mxy = mxy_of(h);
 #pragma unroll
                 for (int e = 0; e < E; ++e) {
@@ -627,8 +631,8 @@ __global__ void __launch_bounds__(kWpThreads * WPP, 1) k_pencil_wp(const __grid_
                 // A(nx, ny) from the tile's ring slot, written before the previous
                 // tile's block barrier
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const double2 A = aslot[b * kTmaMaxTX + 2 * c + h];
+                for (int h = 0; h < PW; ++h) {
+                    const double2 A = aslot[b * kTmaMaxTX + PW * c + h];
 #pragma unroll
                     for (int e = 0; e < E; ++e)
                         pen(v[e], h) = cmul_d(pen(v[e], h), dcmul(A, bz[out_pos<NL, E>(e, t)]));
@@ -658,7 +662,7 @@ __global__ void __launch_bounds__(kWpThreads * WPP, 1) k_pencil_wp(const __grid_
                     }
                 }
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
+                for (int h = 0; h < PW; ++h) {
                     if (h == 0 && has_col0) continue;
                     const long mxy = mxy_of(h);
 #pragma unroll
