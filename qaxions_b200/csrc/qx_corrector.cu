@@ -54,6 +54,12 @@ constexpr int BSITES = BX * BY * BZ;           // 256 sites
 
 __device__ __forceinline__ int wrapi(int i, int n) { return i < 0 ? i + n : (i >= n ? i - n : i); }
 
+// first 128-byte boundary of dynamic shared memory, as an offset from it (a
+// pointer rounded through an integer would make every access generic)
+__device__ __forceinline__ unsigned char* smem_align128(unsigned char* p) {
+    return p + ((128u - ((uint32_t)__cvta_generic_to_shared(p) & 127u)) & 127u);
+}
+
 // offset index o = (dz+1)*9 + (dy+1)*3 + (dx+1)
 __host__ __device__ constexpr int off_dx(int o) { return o % 3 - 1; }
 __host__ __device__ constexpr int off_dy(int o) { return (o / 3) % 3 - 1; }
@@ -316,7 +322,7 @@ __global__ void __launch_bounds__(256, 2) k_conv_tc(const __nv_bfloat16* __restr
     __shared__ uint32_t tmem_slot;
     __shared__ float bs[COUT];
     __shared__ int s_fail;
-    unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_tc) + 127) & ~(uintptr_t)127);
+    unsigned char* base = smem_align128(smem_tc);
     unsigned char* halo = base;
     unsigned char* wsm = base + HALO_BYTES;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -574,7 +580,7 @@ __global__ void __launch_bounds__(256, 1) k_wgrad_tc(const __nv_bfloat16* __rest
     __shared__ __align__(8) uint64_t mbar[2];
     __shared__ uint32_t tmem_slot;
     __shared__ float bred[8][32];
-    unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_w) + 127) & ~(uintptr_t)127);
+    unsigned char* base = smem_align128(smem_w);
     unsigned char* oper[2] = {base, base + wtc::OPER_BYTES};
     unsigned char* dzb = base + 2 * wtc::OPER_BYTES;
     __nv_bfloat16* halo = reinterpret_cast<__nv_bfloat16*>(dzb + wtc::DZ_BYTES);

@@ -69,9 +69,28 @@ template <typename C> __device__ __forceinline__ CPair<C> cscale(CPair<C> u, dec
 template <int SIGN, typename C> __device__ __forceinline__ CPair<C> cmul_si(CPair<C> u) {
     return {cmul_si<SIGN>(u.a), cmul_si<SIGN>(u.b)};
 }
+// u + SIGN i v
+template <int SIGN, typename C> __device__ __forceinline__ C cadd_i(C u, C v) {
+    return SIGN < 0 ? mk<C>(u.x + v.y, u.y - v.x) : mk<C>(u.x - v.y, u.y + v.x);
+}
+template <int SIGN, typename C> __device__ __forceinline__ CPair<C> cadd_i(CPair<C> u, CPair<C> v) {
+    return {cadd_i<SIGN>(u.a, v.a), cadd_i<SIGN>(u.b, v.b)};
+}
+// u + SIGN i k v, one rounding
+template <int SIGN, typename C> __device__ __forceinline__ C cfma_i(C u, C v, decltype(C::x) k) {
+    return SIGN < 0 ? mk<C>(fma(v.y, k, u.x), fma(-v.x, k, u.y)) : mk<C>(fma(-v.y, k, u.x), fma(v.x, k, u.y));
+}
+template <int SIGN, typename C> __device__ __forceinline__ CPair<C> cfma_i(CPair<C> u, CPair<C> v, decltype(C::x) k) {
+    return {cfma_i<SIGN>(u.a, v.a, k), cfma_i<SIGN>(u.b, v.b, k)};
+}
 // pencil h (0 or 1) of a value
-template <typename C> __device__ __forceinline__ C& pen(C& v, int) { return v; }
-template <typename C> __device__ __forceinline__ C& pen(CPair<C>& v, int h) { return h ? v.b : v.a; }
+template <typename C> __device__ __forceinline__ C pen(const C& v, int) { return v; }
+template <typename C> __device__ __forceinline__ C pen(const CPair<C>& v, int h) { return h ? v.b : v.a; }
+template <typename C> __device__ __forceinline__ void pen_set(C& v, int, C w) { v = w; }
+template <typename C> __device__ __forceinline__ void pen_set(CPair<C>& v, int h, C w) {
+    if (h) v.b = w;
+    else v.a = w;
+}
 
 // ---------------------------------------------------------------------------
 // Radix plans (compile time).  Default plan of a length n: n = 2^e:
@@ -172,11 +191,11 @@ template <int SIGN, typename C> __device__ __forceinline__ void dft2(C* a) {
 
 template <int SIGN, typename C> __device__ __forceinline__ void dft4(C* a) {
     C t0 = cadd(a[0], a[2]), t1 = csub(a[0], a[2]);
-    C t2 = cadd(a[1], a[3]), t3 = cmul_si<SIGN>(csub(a[1], a[3]));
+    C t2 = cadd(a[1], a[3]), d = csub(a[1], a[3]);
     a[0] = cadd(t0, t2);
     a[2] = csub(t0, t2);
-    a[1] = cadd(t1, t3);
-    a[3] = csub(t1, t3);
+    a[1] = cadd_i<SIGN>(t1, d);
+    a[3] = cadd_i<-SIGN>(t1, d);
 }
 
 template <int SIGN, typename C> __device__ __forceinline__ void dft3(C* a) {
@@ -184,10 +203,9 @@ template <int SIGN, typename C> __device__ __forceinline__ void dft3(C* a) {
     const C s = cadd(a[1], a[2]);
     const C d = csub(a[1], a[2]);
     const C m = csub(a[0], cscale(s, R(0.5)));
-    const C rot = cmul_si<SIGN>(cscale(d, Consts<R>::sqrt3_2));
     a[0] = cadd(a[0], s);
-    a[1] = cadd(m, rot);
-    a[2] = csub(m, rot);
+    a[1] = cfma_i<SIGN>(m, d, Consts<R>::sqrt3_2);
+    a[2] = cfma_i<-SIGN>(m, d, Consts<R>::sqrt3_2);
 }
 
 template <int SIGN, typename C> __device__ __forceinline__ void dft8(C* a) {
@@ -195,16 +213,17 @@ template <int SIGN, typename C> __device__ __forceinline__ void dft8(C* a) {
     C o[4] = {a[1], a[3], a[5], a[7]};
     dft4<SIGN>(e);
     dft4<SIGN>(o);
-    // o[q] *= W8^q (sign SIGN): W8^1 = h(1 + SIGN i), W8^2 = SIGN i, W8^3 = h(-1 + SIGN i)
-    const C o1 = o[1], o3 = o[3];
-    o[1] = cscale_rsqrt2(cadd(o1, cmul_si<SIGN>(o1)));
-    o[2] = cmul_si<SIGN>(o[2]);
-    o[3] = cscale_rsqrt2(csub(cmul_si<SIGN>(o3), o3));
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        a[q] = cadd(e[q], o[q]);
-        a[q + 4] = csub(e[q], o[q]);
-    }
+    // o[q] *= W8^q (sign SIGN): W8^1 = h(1 + SIGN i), W8^2 = SIGN i, W8^3 = -h(1 - SIGN i)
+    const C o1 = cscale_rsqrt2(cadd_i<SIGN>(o[1], o[1]));
+    const C o3 = cscale_rsqrt2(cadd_i<-SIGN>(o[3], o[3]));
+    a[0] = cadd(e[0], o[0]);
+    a[4] = csub(e[0], o[0]);
+    a[1] = cadd(e[1], o1);
+    a[5] = csub(e[1], o1);
+    a[2] = cadd_i<SIGN>(e[2], o[2]);
+    a[6] = cadd_i<-SIGN>(e[2], o[2]);
+    a[3] = csub(e[3], o3);
+    a[7] = cadd(e[3], o3);
 }
 
 template <int r, int SIGN, typename C> __device__ __forceinline__ void dft(C* a) {
@@ -218,7 +237,10 @@ template <int r, int SIGN, typename C> __device__ __forceinline__ void dft(C* a)
 // ---------------------------------------------------------------------------
 // Stage driver.
 // Acc: shared-memory accessor with `C& operator()(int pos)` for this pencil and
-// a `sync()` that is a barrier over every thread sharing the buffer.
+// a `sync()` that is a barrier over every thread sharing the buffer.  With kSplit
+// it is called as operator()(tp, kc) instead: position tp + kc, tp that of the
+// thread's first value and kc a compile-time offset, in disjoint bits (lengths
+// 2^e), for accessors whose address is not affine in the position.
 // ---------------------------------------------------------------------------
 
 // Butterfly column j of block b of thread t at stage s.  J0 = 1 pairs the
@@ -300,6 +322,15 @@ template <int SIGN, typename C> __device__ __forceinline__ CPair<C> tw_mul(CPair
     return {df_mul(v.a, w, l), df_mul(v.b, w, l)};
 }
 
+// Position held by v[e] in the OUTPUT order of forward stage s (where stage s
+// writes its results); for the last stage this is out_pos.
+template <int L, int E, int s, int J0 = 0> __device__ __forceinline__ int stage_out_pos(int e, int t) {
+    constexpr int r = qx_radix(L, s);
+    constexpr int Ns = qx_span(L, s);
+    const int j = stage_j<L, E, s, J0>(e / r, t);
+    return (j / Ns) * Ns * r + (j % Ns) + (e % r) * Ns;
+}
+
 template <int L, int E, int SIGN, int s, int J0, typename C, typename Acc, typename TW>
 __device__ __forceinline__ void fft_stages(C (&v)[E], Acc& acc, int t, const TW& tw) {
     constexpr int S = qx_nstages(L);
@@ -324,13 +355,22 @@ __device__ __forceinline__ void fft_stages(C (&v)[E], Acc& acc, int t, const TW&
 #pragma unroll
             for (int b = 0; b < nb; ++b) {
                 const int j = stage_j<L, E, s, J0>(b, t);
-                const int idxD = (j / Ns) * Ns * r + (j % Ns);
+                if constexpr (Acc::kSplit) {
 #pragma unroll
-                for (int m = 0; m < r; ++m) acc(idxD + m * Ns) = v[b * r + m];
+                    for (int m = 0; m < r; ++m)
+                        acc(stage_out_pos<L, E, s, J0>(0, t), stage_out_pos<L, E, s, J0>(b * r + m, 0)) = v[b * r + m];
+                } else {
+                    const int idxD = (j / Ns) * Ns * r + (j % Ns);
+#pragma unroll
+                    for (int m = 0; m < r; ++m) acc(idxD + m * Ns) = v[b * r + m];
+                }
             }
             acc.sync();
 #pragma unroll
-            for (int e = 0; e < E; ++e) v[e] = acc(in_pos<L, E, s + 1>(e, t));
+            for (int e = 0; e < E; ++e) {
+                if constexpr (Acc::kSplit) v[e] = acc(t, in_pos<L, E, s + 1>(e, 0));
+                else v[e] = acc(in_pos<L, E, s + 1>(e, t));
+            }
             fft_stages<L, E, SIGN, s + 1, J0>(v, acc, t, tw);
         }
     }
@@ -362,15 +402,6 @@ __device__ __forceinline__ auto tw_src(const C* hi, const C* lo) {
     }
 }
 
-// Position held by v[e] in the OUTPUT order of forward stage s (where stage s
-// writes its results); for the last stage this is out_pos.
-template <int L, int E, int s, int J0 = 0> __device__ __forceinline__ int stage_out_pos(int e, int t) {
-    constexpr int r = qx_radix(L, s);
-    constexpr int Ns = qx_span(L, s);
-    const int j = stage_j<L, E, s, J0>(e / r, t);
-    return (j / Ns) * Ns * r + (j % Ns) + (e % r) * Ns;
-}
-
 // Undo forward stage s (inverse butterfly, then conjugate twiddles), then
 // move on to stage s-1.  Entry: v in stage_out_pos<s> order; exit of the
 // whole chain: v in stage-0 input order (in_pos<L,E,0,J0>).
@@ -391,10 +422,18 @@ __device__ __forceinline__ void ifft_rev_stages(C (&v)[E], Acc& acc, int t, cons
     if constexpr (s > 0) {
         acc.sync();
 #pragma unroll
-        for (int e = 0; e < E; ++e) acc(in_pos<L, E, s>(e, t)) = v[e];
+        for (int e = 0; e < E; ++e) {
+            if constexpr (Acc::kSplit) acc(t, in_pos<L, E, s>(e, 0)) = v[e];
+            else acc(in_pos<L, E, s>(e, t)) = v[e];
+        }
         acc.sync();
 #pragma unroll
-        for (int e = 0; e < E; ++e) v[e] = acc(stage_out_pos<L, E, s - 1, J0>(e, t));
+        for (int e = 0; e < E; ++e) {
+            if constexpr (Acc::kSplit)
+                v[e] = acc(stage_out_pos<L, E, s - 1, J0>(0, t), stage_out_pos<L, E, s - 1, J0>(e, 0));
+            else
+                v[e] = acc(stage_out_pos<L, E, s - 1, J0>(e, t));
+        }
         ifft_rev_stages<L, E, s - 1, J0>(v, acc, t, tw);
     }
 }

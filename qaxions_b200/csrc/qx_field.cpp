@@ -439,10 +439,10 @@ class FieldT final : public Field {
         QX_CUDA(cudaMemsetAsync(vh_.p, 0, vh_.bytes, st_));
         fft_ = std::make_unique<B200FFTBackend<R>>(g_, tw_, &tune_, st_, err_);
         // measured default at 512^3: FP32, the wave-function passes with one warp per
-        // pencil pair (the drift pass with two warps per pair), the half-spectrum
-        // passes with the 8-column tiles; FP64, one warp per pencil in the
-        // wave-function passes and two in the Poisson pass (launch_tma_tx)
-        if (cfg.dim == 3 && cfg.N == 512) tune_.wp = sizeof(R) == 4 ? 3 : 1;
+        // pencil pair, the half-spectrum passes with the 8-column tiles; FP64, one
+        // warp per pencil in the wave-function passes and two in the Poisson pass
+        // (launch_tma_tx)
+        if (cfg.dim == 3 && cfg.N == 512) tune_.wp = 1;
         consult_tune_cache();
         // drift chain: phase counters (as many as 8-column slabs need)
         chain_n_ = Ops<R>::chain_slabs(g_.N, g_.dim, g_.B, 1);

@@ -44,6 +44,7 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 // row's threads all sit in one warp (qx_row_threads(N) divides 32), so its
 // exchanges only need a warp barrier; `mask` names the warp's existing lanes.
 template <typename C> struct RowAcc {
+    static constexpr bool kSplit = false;
     C* base;
     unsigned mask;
     __device__ __forceinline__ C& operator()(int p) const { return base[p + (p >> 4)]; }
@@ -75,6 +76,7 @@ template <int N> __host__ __device__ constexpr int row_pair_idx(int e, int h) {
 
 // column of a strided tile: element p of this pencil at base[p * pitch]
 template <typename C> struct ColAcc {
+    static constexpr bool kSplit = false;
     C* base;
     int pitch;
     __device__ __forceinline__ C& operator()(int p) const { return base[p * pitch]; }
@@ -302,10 +304,19 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
 
+// first address at or above p on an A-byte boundary of shared memory, formed as
+// an offset so that the compiler still sees a shared-memory pointer (rounding
+// the pointer through an integer makes every access through it a generic one;
+// with shared accesses the 512^3 FP32 passes took, us: z drift 806 -> 676, y
+// forward 403 -> 379, z Poisson 390 -> 375, x c2r + kick 600 -> 576)
+template <uint32_t A> __device__ __forceinline__ unsigned char* smem_align(unsigned char* p) {
+    return p + ((A - ((uint32_t)__cvta_generic_to_shared(p) & (A - 1))) & (A - 1));
+}
+
 // per-warp staging buffer after the P row buffers (16-byte aligned for cp.async)
 template <int N, typename C> __device__ __forceinline__ C* x_stage_ptr(C* row_buf, int stage_elems) {
     C* end = row_buf - threadIdx.y * row_smem_elems(N) + blockDim.y * row_smem_elems(N);
-    return reinterpret_cast<C*>((reinterpret_cast<uintptr_t>(end) + 15) & ~(uintptr_t)15) + threadIdx.y * stage_elems;
+    return reinterpret_cast<C*>(smem_align<16>(reinterpret_cast<unsigned char*>(end))) + threadIdx.y * stage_elems;
 }
 
 enum XFwdMode { XF_PLAIN = 0, XF_KICK = 1 };

@@ -173,6 +173,7 @@ template <typename C> __device__ __forceinline__ void ld_cg_pair(const C* row, i
 
 // column of a strided unit: element p of slot c at base[p * pitch]
 template <typename P> struct UnitColAcc {
+    static constexpr bool kSplit = false;
     P* base;
     int pitch, bar;
     __device__ __forceinline__ P& operator()(int p) const { return base[p * pitch]; }
@@ -252,7 +253,7 @@ __device__ __forceinline__ void mx_pencil_unit(const MGroup<R>& G, long l, int t
         for (int h = 0; h < PW; ++h) {
             const double2 A = valid ? G.axy[(long)y * N + x + h] : make_double2(0.0, 0.0);
 #pragma unroll
-            for (int e = 0; e < E; ++e) pen(v[e], h) = cmul_d(pen(v[e], h), dcmul(A, tb.bz[out_pos<N, E>(e, t)]));
+            for (int e = 0; e < E; ++e) pen_set(v[e], h, cmul_d(pen(v[e], h), dcmul(A, tb.bz[out_pos<N, E>(e, t)])));
         }
     } else {
         SArgs<R> sa;
@@ -279,7 +280,7 @@ __device__ __forceinline__ void mx_pencil_unit(const MGroup<R>& G, long l, int t
                     const R al = R(0.5) * (gA + gB), be = R(0.5) * (gA - gB);
                     P mv = mb[((N - p) % N) * PITCH];
                     const C cm = cconj(pen(mv, 0));
-                    pen(v[e], 0) = cadd(cscale(pen(v[e], 0), al), cscale(cm, be));
+                    pen_set(v[e], 0, cadd(cscale(pen(v[e], 0), al), cscale(cm, be)));
                 }
             }
         }
@@ -291,7 +292,7 @@ __device__ __forceinline__ void mx_pencil_unit(const MGroup<R>& G, long l, int t
 #pragma unroll
             for (int e = 0; e < E; ++e) {
                 const long nz = signed_mode(out_pos<N, E>(e, t), N);
-                pen(v[e], h) = cscale(pen(v[e], h), pois_mult<R>(mxy + nz * nz, sa));
+                pen_set(v[e], h, cscale(pen(v[e], h), pois_mult<R>(mxy + nz * nz, sa)));
             }
         }
     }

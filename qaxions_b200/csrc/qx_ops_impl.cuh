@@ -361,7 +361,7 @@ static long launch_wp(const typename Ops<R>::SP& a, int NZ, int outer, int penci
         set_smem(kern, smem);
         long grid = (long)sm_count();
         if (grid > s.n_tiles) grid = s.n_tiles;
-        kern<<<(unsigned)grid, dim3(32 * WPP, kWpThreads / 32), smem, st>>>(tm, s);
+        kern<<<(unsigned)grid, dim3(kWpThreads * WPP), smem, st>>>(tm, s);
         QX_LAUNCH_CHECK();
         return grid;
     } else {

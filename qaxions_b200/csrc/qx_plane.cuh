@@ -77,6 +77,7 @@ __host__ __device__ constexpr bool plane_fits(int N, int real_bytes) {
 
 // column unit of the plane: element p of its pencils; NT threads share it
 template <typename P, typename C, int PITCH, int NT, bool ALL> struct PColAcc {
+    static constexpr bool kSplit = false;
     C* base;
     __device__ __forceinline__ P& operator()(int p) const { return *reinterpret_cast<P*>(base + p * PITCH); }
     __device__ __forceinline__ void sync() const {
@@ -86,6 +87,7 @@ template <typename P, typename C, int PITCH, int NT, bool ALL> struct PColAcc {
 };
 // row of the plane (its threads sit in one warp)
 template <typename G> struct PRowAcc {
+    static constexpr bool kSplit = false;
     using C = typename G::C;
     C* base;
     __device__ __forceinline__ C& operator()(int p) const { return base[G::xpad(p)]; }
@@ -436,6 +438,7 @@ template <int N, typename R, int UX> struct ColGeo {
 };
 
 template <typename P> struct ColTileAcc {
+    static constexpr bool kSplit = false;
     P* base;
     int pitch, pad, nt;  // row p at base[(p + (pad ? p >> 3 : 0)) * pitch]; nt threads share the buffer
     __device__ __forceinline__ P& operator()(int p) const { return base[(p + (pad ? (p >> 3) : 0)) * pitch]; }
@@ -498,7 +501,7 @@ __global__ void __launch_bounds__((ColGeo<N, R, UX>::NT + (OP == OP_POISSON && D
 #pragma unroll
         for (int h = 0; h < PW; ++h)
 #pragma unroll
-            for (int e = 0; e < E; ++e) pen(v[e], h) = cmul_d(pen(v[e], h), dcmul(A[h], bz[out_pos<N, E>(e, t)]));
+            for (int e = 0; e < E; ++e) pen_set(v[e], h, cmul_d(pen(v[e], h), dcmul(A[h], bz[out_pos<N, E>(e, t)])));
     } else {
         const bool col0 = tile0 && u == 0 && own0;  // pencil 0 is column 0, finished by this thread
         if (tile0 && own0) {
@@ -519,7 +522,7 @@ __global__ void __launch_bounds__((ColGeo<N, R, UX>::NT + (OP == OP_POISSON && D
                 const long mA = ny * ny + nz * nz, mB = mA + (long)(N / 2) * (N / 2);
                 const R gA = pois_mult<R>(mA, s), gB = pois_mult<R>(mB, s);
                 const C cm = cconj(mir[(N - p) % N]);
-                pen(v[e], 0) = cadd(cscale(pen(v[e], 0), R(0.5) * (gA + gB)), cscale(cm, R(0.5) * (gA - gB)));
+                pen_set(v[e], 0, cadd(cscale(pen(v[e], 0), R(0.5) * (gA + gB)), cscale(cm, R(0.5) * (gA - gB))));
             }
         }
         const bool has_col0 = tile0 && u == 0;
@@ -531,7 +534,7 @@ __global__ void __launch_bounds__((ColGeo<N, R, UX>::NT + (OP == OP_POISSON && D
 #pragma unroll
             for (int e = 0; e < E; ++e) {
                 const int nz = signed_mode(out_pos<N, E>(e, t), N);
-                pen(v[e], h) = cscale(pen(v[e], h), pois_mult<R>(mxy + (long)nz * nz, s));
+                pen_set(v[e], h, cscale(pen(v[e], h), pois_mult<R>(mxy + (long)nz * nz, s)));
             }
         }
     }

@@ -176,6 +176,7 @@ __device__ __forceinline__ void named_barrier(int id, int nthreads) {
 // pencil group c of a tile: element p at base[p * pitch + c] (plain) or at
 // base[p * 8 + (c ^ (p & 7))] (swizzled 128-byte rows of 8 pairs)
 template <typename P, bool SWZ> struct TileAcc {
+    static constexpr bool kSplit = false;
     P* base;
     int c, pitch;
     __device__ __forceinline__ P& operator()(int p) const {
@@ -215,8 +216,8 @@ __global__ void __launch_bounds__((tma_block_threads<N, R, PW, TXF>()), (tma_blo
     const uint32_t tile_bytes = (uint32_t)((size_t)N * TX * sizeof(C));
     const long tile_elems = (long)(align1k(tile_bytes) / sizeof(C));
     // tiles on 128-byte boundaries, 1024 for the 128-byte swizzle
-    constexpr uintptr_t BA = SWZ ? 1023 : 127;
-    C* bufs = reinterpret_cast<C*>((reinterpret_cast<uintptr_t>(smem_raw) + BA) & ~BA);
+    constexpr uint32_t BA = SWZ ? 1023 : 127;
+    C* bufs = reinterpret_cast<C*>(smem_align<BA + 1>(smem_raw));
     C* tws = bufs + s.nbuf * tile_elems;
     C* tws_lo = tws + N;
     double2* bz = reinterpret_cast<double2*>(tws_lo + N);
@@ -333,12 +334,14 @@ __global__ void __launch_bounds__((tma_block_threads<N, R, PW, TXF>()), (tma_blo
                 // (staged before the previous tile's store barrier; a multi-stage
                 // forward transform has synchronised the block since)
                 if constexpr (qx_nstages(NL) == 1) __syncthreads();
+                double2 A[PW];
 #pragma unroll
-                for (int h = 0; h < PW; ++h) {
-                    const double2 A = aslot[b * kTmaMaxTX + PW * c + h];
+                for (int h = 0; h < PW; ++h) A[h] = aslot[b * kTmaMaxTX + PW * c + h];
 #pragma unroll
-                    for (int e = 0; e < E; ++e)
-                        pen(v[e], h) = cmul_d(pen(v[e], h), dcmul(A, bz[out_pos<NL, E>(e, t)]));
+                for (int e = 0; e < E; ++e) {
+                    const double2 B = bz[out_pos<NL, E>(e, t)];
+#pragma unroll
+                    for (int h = 0; h < PW; ++h) pen_set(v[e], h, cmul_d(pen(v[e], h), dcmul(A[h], B)));
                 }
             } else {
                 SArgs<R> sa;
@@ -363,7 +366,7 @@ __global__ void __launch_bounds__((tma_block_threads<N, R, PW, TXF>()), (tma_blo
                             const long mA = np * np, mB = mA + (long)(N / 2) * (N / 2);
                             const R gA = pois_mult<R>(mA, sa), gB = pois_mult<R>(mB, sa);
                             const C cm = cconj(pen(acc((N - p) % N), 0));
-                            pen(v[e], 0) = cadd(cscale(pen(v[e], 0), R(0.5) * (gA + gB)), cscale(cm, R(0.5) * (gA - gB)));
+                            pen_set(v[e], 0, cadd(cscale(pen(v[e], 0), R(0.5) * (gA + gB)), cscale(cm, R(0.5) * (gA - gB))));
                         }
                     }
                 }
@@ -374,7 +377,7 @@ __global__ void __launch_bounds__((tma_block_threads<N, R, PW, TXF>()), (tma_blo
 #pragma unroll
                     for (int e = 0; e < E; ++e) {
                         const int nz = signed_mode(out_pos<NL, E>(e, t), N);
-                        pen(v[e], h) = cscale(pen(v[e], h), pois_mult<R>(mxy + (long)nz * nz, sa));
+                        pen_set(v[e], h, cscale(pen(v[e], h), pois_mult<R>(mxy + (long)nz * nz, sa)));
                     }
                 }
             }
@@ -387,7 +390,7 @@ __global__ void __launch_bounds__((tma_block_threads<N, R, PW, TXF>()), (tma_blo
                 if constexpr (qx_nstages(NL) == 1) __syncthreads();
                 if (c0ext) {
 #pragma unroll
-                    for (int e = 0; e < E; ++e) pen(v[e], 0) = col0[in_pos<NL, E, 0>(e, t)];
+                    for (int e = 0; e < E; ++e) pen_set(v[e], 0, col0[in_pos<NL, E, 0>(e, t)]);
                 }
             }
         }
@@ -468,27 +471,33 @@ __global__ void __launch_bounds__((tma_block_threads<N, R, PW, TXF>()), (tma_blo
 // stores to the tensor copy use the identity rows.
 // ---------------------------------------------------------------------------
 
-// barrier over the WPP warps that share pencil pair c (named barrier 1 + c)
-template <int WPP> __device__ __forceinline__ void pair_sync(int c) {
+// barrier over the WPP warps that share pencil unit c (named barrier 1 + c)
+template <int WPP> __device__ __forceinline__ void unit_sync(int c) {
     if constexpr (WPP == 1) __syncwarp();
     else named_barrier(1 + c, 32 * WPP);
 }
-// a pencil pair's element p in the tensor copy's row p of a swizzled tile
-template <typename P, int WPP = 1> struct SwzRowAcc {
-    P* base;
+// Pencil unit c of a swizzled tile.  Element p sits in row r, chunk c ^ (r & 7), with
+// r = p in the tensor copy (SIGMA = false) and r = sigma(p) = p ^ ((p >> 3) & 7) in the
+// exchanges.  The byte offset (r << 7) + ((c ^ (r & 7)) << 4) is XOR-linear in the
+// bits of p, so for p = tp + kc (disjoint bits) it is the offset of tp, one
+// register per access pattern, with compile-time bits of kc XORed in below 1 KB
+// and added above: no per-element address registers.  `tile` is a byte offset from
+// `bufs` that changes from tile to tile, which keeps the compiler from hoisting
+// the addresses out of the tile loop.
+template <typename V, int WPP, bool SIGMA> struct WarpAcc {
+    static constexpr bool kSplit = true;
+    unsigned char* bufs;
+    uint32_t tile;
     int c;
-    __device__ __forceinline__ P& operator()(int p) const { return base[p * 8 + (c ^ (p & 7))]; }
-    __device__ __forceinline__ void sync() const { pair_sync<WPP>(c); }
-};
-// the same slots with the exchange rows sigma(p)
-template <typename P, int WPP = 1> struct WarpXAcc {
-    P* base;
-    int c;
-    __device__ __forceinline__ P& operator()(int p) const {
-        const int r = p ^ ((p >> 3) & 7);
-        return base[r * 8 + (c ^ (r & 7))];
+    __device__ __forceinline__ static constexpr uint32_t lin(int p) {
+        const int r = SIGMA ? p ^ ((p >> 3) & 7) : p;
+        return ((uint32_t)r << 7) | ((uint32_t)(r & 7) << 4);
     }
-    __device__ __forceinline__ void sync() const { pair_sync<WPP>(c); }
+    __device__ __forceinline__ V& operator()(int tp, int kc) const {
+        const uint32_t a = tile + (lin(tp) ^ ((uint32_t)c << 4));
+        return *reinterpret_cast<V*>(bufs + ((a ^ (lin(kc) & 0x3ffu)) + (lin(kc) & ~0x3ffu)));
+    }
+    __device__ __forceinline__ void sync() const { unit_sync<WPP>(c); }
 };
 
 // tile columns: 8 pencil units of 16 bytes (a pair of FP32 pencils or one FP64
@@ -498,14 +507,15 @@ constexpr int kWpThreads = 256;  // 8 warps, one pencil unit each
 
 __host__ __device__ constexpr bool wp_supported(int N) { return N == 256 || N == 512; }
 
-// WPP warps per pencil pair: WPP = 1 keeps E = N/32 values of each pencil per
-// lane (exchanges under __syncwarp); WPP = 2 (N = 512, the wave-function
-// passes) splits a pair over two warps with E = N/64, halving the registers so
-// that 16 warps fit on an SM, and synchronises the pair's exchanges with a
-// 64-thread named barrier.  The exchange rows are the same; with 64 threads
-// and radix-8 stages every exchange stays conflict-free (each 8-lane phase of
-// an access meets 8 distinct rows mod 8 after sigma).
-// blockDim = (32 WPP, 8): thread t = threadIdx.x of pencil pair c = threadIdx.y
+// WPP warps per pencil unit, E = N / (32 WPP) values of each pencil per thread:
+// WPP = 1 is 8 warps per SM whose exchanges need __syncwarp only; WPP = 2 (N =
+// 512) is 16 warps with half the registers, a unit's exchanges under a 64-thread
+// named barrier.  The exchange rows are the same and conflict-free in both.
+// Measured at 512^3 FP32 (us, WPP 1 / 2): z drift 676 / 692, y forward 379 / 396.
+// Several units per warp (a twiddle load then touches 16 or 8 table entries, the
+// exchanges synchronise 2 or 4 warps) measured the same or slower (z drift 692 /
+// 686 with two units, 715 with four), so shared-memory wavefronts of the twiddles
+// are not what bounds it.
 template <int N, typename R, int OP, bool DF, int PLAN = 0, int WPP = 1>
 __global__ void __launch_bounds__(kWpThreads * WPP, 1) k_pencil_wp(const __grid_constant__ CUtensorMap tm, TArgs<R> s) {
     using C = cx_t<R>;
@@ -523,12 +533,12 @@ __global__ void __launch_bounds__(kWpThreads * WPP, 1) k_pencil_wp(const __grid_
     __shared__ __align__(8) uint64_t mbar[8];
     __shared__ int s_abort;
     __shared__ double red[32];
-    const int t = threadIdx.x, c = threadIdx.y;
-    const int tid = threadIdx.x + TPP * threadIdx.y;
+    const int tid = threadIdx.x;
+    const int c = tid / TPP, t = tid % TPP;  // pencil unit and thread within it
     const int nthr = kWpThreads * WPP;
     const uint32_t tile_bytes = (uint32_t)((size_t)N * TX * sizeof(C));
     const long tile_elems = (long)(align1k(tile_bytes) / sizeof(C));
-    C* bufs = reinterpret_cast<C*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    C* bufs = reinterpret_cast<C*>(smem_align<1024>(smem_raw));
     C* tws = bufs + s.nbuf * tile_elems;
     C* tws_lo = tws + N;
     double2* bz = reinterpret_cast<double2*>(tws_lo + N);
@@ -587,8 +597,9 @@ __global__ void __launch_bounds__(kWpThreads * WPP, 1) k_pencil_wp(const __grid_
         const int x0 = (int)(id % s.tiles_x) * TX;
         const int o = (int)(id / s.tiles_x);
         const int xb = x0 + PW * c;
-        SwzRowAcc<P, WPP> io{reinterpret_cast<P*>(tile), c};
-        WarpXAcc<P, WPP> acc{reinterpret_cast<P*>(tile), c};
+        const uint32_t tile_off = (uint32_t)b * (uint32_t)(tile_elems * sizeof(C));
+        WarpAcc<P, WPP, false> io{reinterpret_cast<unsigned char*>(bufs), tile_off, c};
+        WarpAcc<P, WPP, true> acc{reinterpret_cast<unsigned char*>(bufs), tile_off, c};
         const long id_next = id + gridDim.x;
         const bool a_copy = OP == OP_DRIFT && tid < TX && id_next < s.n_tiles;
         if (a_copy) {
@@ -598,11 +609,11 @@ __global__ void __launch_bounds__(kWpThreads * WPP, 1) k_pencil_wp(const __grid_
         P v[E];
         if constexpr (OP == OP_INV) {
 #pragma unroll
-            for (int e = 0; e < E; ++e) v[e] = io(out_pos<NL, E>(e, t));
+            for (int e = 0; e < E; ++e) v[e] = io(out_pos<NL, E>(0, t), out_pos<NL, E>(e, 0));
             ifft_pencil_rev<NL, E>(v, acc, t, tw_src<DF>(tws, tws_lo));
         } else {
 #pragma unroll
-            for (int e = 0; e < E; ++e) v[e] = io(in_pos<NL, E, 0>(e, t));
+            for (int e = 0; e < E; ++e) v[e] = io(t, in_pos<NL, E, 0>(e, 0));
             fft_pencil<NL, E, -1>(v, acc, t, tw_src<DF>(tws, tws_lo));
         }
         auto mxy_of = [&](int h) {
@@ -630,12 +641,16 @@ __global__ void __launch_bounds__(kWpThreads * WPP, 1) k_pencil_wp(const __grid_
             if constexpr (OP == OP_DRIFT) {
                 // A(nx, ny) from the tile's ring slot, written before the previous
                 // tile's block barrier
+                double2 A[PW];
 #pragma unroll
-                for (int h = 0; h < PW; ++h) {
-                    const double2 A = aslot[b * kTmaMaxTX + PW * c + h];
+                for (int h = 0; h < PW; ++h) A[h] = aslot[b * kTmaMaxTX + PW * c + h];
 #pragma unroll
-                    for (int e = 0; e < E; ++e)
-                        pen(v[e], h) = cmul_d(pen(v[e], h), dcmul(A, bz[out_pos<NL, E>(e, t)]));
+                for (int e = 0; e < E; ++e) {
+                    const double2 B = bz[out_pos<NL, E>(e, t)];
+#pragma unroll
+                    for (int h = 0; h < PW; ++h) pen_set(v[e], h, cmul_d(pen(v[e], h), dcmul(A[h], B)));
+                    // (keeps the factors of later positions from being formed early: registers)
+                    if (PW == 2) asm volatile("" ::: "memory");
                 }
             } else {
                 SArgs<R> sa;
@@ -645,20 +660,21 @@ __global__ void __launch_bounds__(kWpThreads * WPP, 1) k_pencil_wp(const __grid_
                     // 3D: column 0 is finished by k_poisson_col0; keep its forward result
 #pragma unroll
                     for (int e = 0; e < E; ++e) col0[out_pos<NL, E>(e, t)] = pen(v[e], 0);
-                } else if (has_col0 && !s.col0_external) {
-                    // 2D: the mirror -k_y of column 0 lies in the same pencil (this pair's)
-                    pair_sync<WPP>(c);
+                }
+                if (has_col0 && !s.col0_external) {
+                    // 2D: the mirror -k_y of column 0 lies in the same pencil
+                    unit_sync<WPP>(c);
 #pragma unroll
-                    for (int e = 0; e < E; ++e) acc(out_pos<NL, E>(e, t)) = v[e];
-                    pair_sync<WPP>(c);
+                    for (int e = 0; e < E; ++e) acc(out_pos<NL, E>(0, t), out_pos<NL, E>(e, 0)) = v[e];
+                    unit_sync<WPP>(c);
 #pragma unroll
                     for (int e = 0; e < E; ++e) {
                         const int p = out_pos<NL, E>(e, t);
                         const long np = signed_mode(p, N);
                         const long mA = np * np, mB = mA + (long)(N / 2) * (N / 2);
                         const R gA = pois_mult<R>(mA, sa), gB = pois_mult<R>(mB, sa);
-                        const C cm = cconj(pen(acc((N - p) % N), 0));
-                        pen(v[e], 0) = cadd(cscale(pen(v[e], 0), R(0.5) * (gA + gB)), cscale(cm, R(0.5) * (gA - gB)));
+                        const C cm = cconj(pen(acc((N - p) % N, 0), 0));
+                        pen_set(v[e], 0, cadd(cscale(pen(v[e], 0), R(0.5) * (gA + gB)), cscale(cm, R(0.5) * (gA - gB))));
                     }
                 }
 #pragma unroll
@@ -668,7 +684,7 @@ __global__ void __launch_bounds__(kWpThreads * WPP, 1) k_pencil_wp(const __grid_
 #pragma unroll
                     for (int e = 0; e < E; ++e) {
                         const int nz = signed_mode(out_pos<NL, E>(e, t), N);
-                        pen(v[e], h) = cscale(pen(v[e], h), pois_mult<R>(mxy + (long)nz * nz, sa));
+                        pen_set(v[e], h, cscale(pen(v[e], h), pois_mult<R>(mxy + (long)nz * nz, sa)));
                     }
                 }
             }
@@ -677,20 +693,20 @@ __global__ void __launch_bounds__(kWpThreads * WPP, 1) k_pencil_wp(const __grid_
                 // the stash was written by other threads of this pencil pair in another
                 // order; the inverse's exchanges synchronised the pair since
 #pragma unroll
-                for (int e = 0; e < E; ++e) pen(v[e], 0) = col0[in_pos<NL, E, 0>(e, t)];
+                for (int e = 0; e < E; ++e) pen_set(v[e], 0, col0[in_pos<NL, E, 0>(e, t)]);
             }
         }
 
         if (a_copy) cp_async_wait_all();
         if (store) {
-            // the finished pencil pair -> its slots (identity rows) -> tensor store
-            pair_sync<WPP>(c);
+            // the finished pencils -> their slots (identity rows) -> tensor store
+            unit_sync<WPP>(c);
             if constexpr (OP == OP_FWD) {
 #pragma unroll
-                for (int e = 0; e < E; ++e) io(out_pos<NL, E>(e, t)) = v[e];
+                for (int e = 0; e < E; ++e) io(out_pos<NL, E>(0, t), out_pos<NL, E>(e, 0)) = v[e];
             } else {
 #pragma unroll
-                for (int e = 0; e < E; ++e) io(in_pos<NL, E, 0>(e, t)) = v[e];
+                for (int e = 0; e < E; ++e) io(t, in_pos<NL, E, 0>(e, 0)) = v[e];
             }
             fence_proxy_async();
             __syncthreads();

@@ -136,6 +136,7 @@ template <int N, typename R, int PW, int TXF> __host__ __device__ constexpr bool
 // tile accessor of a compute group: plain indexing, FFT exchanges
 // synchronised by the group's own named barrier
 template <typename P> struct GroupAcc {
+    static constexpr bool kSplit = false;
     P* base;
     int c, pitch, bar_id, nthr;
     __device__ __forceinline__ P& operator()(int p) const { return base[p * pitch + c]; }
@@ -170,7 +171,7 @@ __global__ void __launch_bounds__((yzy_block_threads<N, R, PW, TXF>()), 1)
     __shared__ int s_abort[2];  // per compute group, written by its own threads only
     const int tid = threadIdx.x;
     const long G = gridDim.x;
-    C* bufs = reinterpret_cast<C*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~(uintptr_t)127);
+    C* bufs = reinterpret_cast<C*>(smem_align<128>(smem_raw));
     C* tws = bufs + s.nbuf * tile_elems;
     C* tws_lo = tws + N;
     double2* bz = reinterpret_cast<double2*>(tws_lo + N);
@@ -366,7 +367,7 @@ __global__ void __launch_bounds__((yzy_block_threads<N, R, PW, TXF>()), 1)
                 for (int e = 0; e < E; ++e) {
                     const double2 bze = bz[out_pos<N, E>(e, t)];
 #pragma unroll
-                    for (int h = 0; h < PW; ++h) pen(v[e], h) = cmul_d(pen(v[e], h), dcmul(A[h], bze));
+                    for (int h = 0; h < PW; ++h) pen_set(v[e], h, cmul_d(pen(v[e], h), dcmul(A[h], bze)));
                 }
             }
             if (ph != 0) ifft_pencil_rev<N, E>(v, acc, t, tw);
