@@ -185,6 +185,19 @@ std::vector<int> spectrum_bin_table(int dim, int N, int mode, int nbins) {
     return tab;
 }
 
+std::vector<int> spectrum_thresholds(const std::vector<int>& tab, int nbins) {
+    long first = 0, end = (long)tab.size();
+    while (first < end && tab[first] < 0) ++first;
+    while (end > first && tab[end - 1] < 0) --end;
+    std::vector<int> T(nbins + 1, (int)end);
+    int b = 0;
+    for (long M = first; M < end; ++M) {
+        if (tab[M] < b - 1 || tab[M] >= nbins) throw std::logic_error("spectrum bins are not sorted");
+        while (b <= tab[M]) T[b++] = (int)M;
+    }
+    return T;
+}
+
 std::vector<double> spectrum_k_axis(int N, int mode, int nbins, double L) {
     const double dk = kTwoPi / L;
     const int nmax = N / 2;
@@ -246,14 +259,6 @@ template <typename R> void B200FFTBackend<R>::forward_c2c(void* data) {
     Ops<R>::x_fwd(g_.N, a, false, *tune_, st_);
     if (g_.dim == 3) Ops<R>::y_pass(g_.N, g_.B * g_.N, sp0<R>(err_, g_, d, tw_, g_.N, *tune_), -1, *tune_, st_);
     Ops<R>::la_pass(g_.N, sp0<R>(err_, g_, d, tw_, g_.N, *tune_), OP_FWD, *tune_, st_);
-}
-
-template <typename R> void B200FFTBackend<R>::forward_c2c_partial(const C* in, C* out) {
-    auto a = xp0<R>(g_, tw_);
-    a.in = in;
-    a.out = out;
-    Ops<R>::x_fwd(g_.N, a, false, *tune_, st_);
-    if (g_.dim == 3) Ops<R>::y_pass(g_.N, g_.B * g_.N, sp0<R>(err_, g_, out, tw_, g_.N, *tune_), -1, *tune_, st_);
 }
 
 template <typename R> void B200FFTBackend<R>::backward_c2c(void* data) {
@@ -739,14 +744,20 @@ class FieldT final : public Field {
         }
         single_box("measure");
         // computeEnergy's rhomax (src/meas.cxx:30), without overwriting V
-        auto rr = reduce(RED_RHO);
-        rhomax_ = rr[1] / (rr[0] / (double)g_.S);
-        r.rhomax = rhomax_;
         ensure_V();
-        vmax_ = reduce(RED_VABS)[1];
+        if (mask & MEAS_ENERGY) {
+            const Diag d = diagnostics();
+            rhomax_ = d.rhomax / (d.rho / (double)g_.S);
+            vmax_ = d.vmax;
+            mass_energy_of(d, &r.mass, &r.energy, &r.kinetic, &r.potential);
+        } else {
+            auto rr = reduce(RED_RHO);
+            rhomax_ = rr[1] / (rr[0] / (double)g_.S);
+            vmax_ = reduce(RED_VABS)[1];
+        }
         vmax_stale_ = false;
+        r.rhomax = rhomax_;
         r.vmax = vmax_;
-        if (mask & MEAS_ENERGY) mass_energy(&r.mass, &r.energy, &r.kinetic, &r.potential);
         const std::string d = dir ? dir : "";
         auto fname = [&](const char* stem, const char* ext) {
             std::ostringstream o;
@@ -913,28 +924,39 @@ class FieldT final : public Field {
         if (!v_current_) updatePotential();
     }
 
-    void mass_energy(double* M, double* E, double* K, double* W) override {
-        const double dV = std::pow(cfg_.L / g_.N, g_.dim);
-        const double m = reduce(RED_RHO)[0] * dV;
+    // sums of the current psi and V in one read of psi per axis (Ops::energy)
+    struct Diag {
+        double rho, rhomax, vrho, vmax, kin;
+    };
+    Diag diagnostics() {
         ensure_V();
-        const double w = 0.5 * dV * reduce(RED_VRHO)[0];
-        // kinetic: 1/2 dV/S sum k^2 |psi^|^2 with the last axis fused into the reduction
-        mpsi_.alloc(sizeof(C) * g_.S);
-        fft_->forward_c2c_partial(psi(), mpsi_.as<C>());
-        auto s = sp(mpsi_.as<C>(), g_.N);
-        const long cap = Ops<R>::la_blocks(g_.N, g_.N, g_.dim, OP_KIN, tune_);
-        kin_.alloc(sizeof(double) * (cap + 1));
-        s.partial = kin_.as<double>();
-        const long nblk = Ops<R>::la_pass(g_.N, s, OP_KIN, tune_, st_);
-        Misc<R>::fold_sum(kin_.as<double>(), nblk, redout_.as<double>(), st_);
-        double ks = 0.0;
-        QX_CUDA(cudaMemcpyAsync(&ks, redout_.p, sizeof(double), cudaMemcpyDeviceToHost, st_));
+        const long cap = Ops<R>::energy_blocks();
+        kin_.alloc(sizeof(double) * (7 * cap + 7));
+        double* part = kin_.as<double>();
+        auto a = xp();
+        a.in = psi();
+        a.Vin = V();
+        long n[3];
+        Ops<R>::energy(g_.N, a, sp(psi(), g_.N), part, n, tune_, st_);
+        fold_energy(part, cap, n, part + 7 * cap, st_);
+        double h[7];
+        QX_CUDA(cudaMemcpyAsync(h, part + 7 * cap, sizeof(h), cudaMemcpyDeviceToHost, st_));
         QX_CUDA(cudaStreamSynchronize(st_));
-        const double kin = 0.5 * dV / (double)g_.S1 * dk() * dk() * ks;
+        return {h[0], h[1], h[2], h[3], h[4] + h[5] + h[6]};
+    }
+    void mass_energy_of(const Diag& d, double* M, double* E, double* K, double* W) const {
+        const double dV = std::pow(cfg_.L / g_.N, g_.dim);
+        const double m = d.rho * dV, w = 0.5 * dV * d.vrho;
+        // 1/2 dV/S sum k^2 |psi^|^2; a transform along one axis carries 1/N of the full one's S
+        const double kin = 0.5 * dV / (double)g_.N * dk() * dk() * d.kin;
         if (M) *M = m;
         if (K) *K = kin;
         if (W) *W = w;
         if (E) *E = kin + w;
+    }
+
+    void mass_energy(double* M, double* E, double* K, double* W) override {
+        mass_energy_of(diagnostics(), M, E, K, W);
     }
 
     void spectrum(int source, int mode, int nbins, double* k, double* P, long long* count) override {
@@ -945,7 +967,7 @@ class FieldT final : public Field {
         const long key = ((long)mode << 20) | nbins;
         auto it = bintab_.find(key);
         if (it == bintab_.end()) {
-            auto tab = spectrum_bin_table(g_.dim, g_.N, mode, nbins);
+            auto tab = spectrum_thresholds(spectrum_bin_table(g_.dim, g_.N, mode, nbins), nbins);
             auto buf = std::make_unique<DevBuf>();
             buf->alloc(sizeof(int) * tab.size());
             QX_CUDA(cudaMemcpy(buf->p, tab.data(), sizeof(int) * tab.size(), cudaMemcpyHostToDevice));
@@ -965,12 +987,12 @@ class FieldT final : public Field {
         }
         y_fwd(mvh_.as<C>(), g_.N / 2);
         Ops<R>::la_pass(g_.N, sp(mvh_.as<C>(), g_.N / 2), OP_FWD, tune_, st_);
-        const int nblk_max = 296;
+        const int nblk_max = kSpecBlocks;
         specP_.alloc(sizeof(double) * (size_t)nblk_max * nbins + sizeof(double) * nbins);
         specC_.alloc(sizeof(long long) * (size_t)nblk_max * nbins + sizeof(long long) * nbins);
         double* partP = specP_.as<double>();
         long long* partC = specC_.as<long long>();
-        const int nblk = Misc<R>::spectrum_bin(mvh_.as<C>(), g_.dim, g_.N, it->second->as<int>(), nbins, partP,
+        const int nblk = Misc<R>::spectrum_bin(mvh_.as<C>(), g_.dim, g_.N, it->second->as<int>(), mode, nbins, partP,
                                                partC, st_);
         double* outP = partP + (size_t)nblk_max * nbins;
         long long* outC = partC + (size_t)nblk_max * nbins;

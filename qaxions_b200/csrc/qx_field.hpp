@@ -98,9 +98,6 @@ class B200FFTBackend : public FFTBackend {
     size_t sites() const override { return (size_t)g_.S; }
     size_t ksites() const override { return (size_t)g_.hsites; }
     ptrdiff_t global_N() const override { return g_.N; }
-    // out-of-place forward c2c along all axes except the last, used by the
-    // kinetic-energy measurement (last axis fused with the reduction)
-    void forward_c2c_partial(const C* in, C* out);
 
   private:
     Geometry g_;
@@ -288,6 +285,8 @@ void unpack_half(int dim, int N, const double* packed, double* fftw_half);
 
 // spectrum bin of every integer |n|^2 (mode 0 reference shells, 1 linear, 2 log)
 std::vector<int> spectrum_bin_table(int dim, int N, int mode, int nbins);
+// the sorted bins of such a table as thresholds: bin b holds T[b] <= |n|^2 < T[b + 1]
+std::vector<int> spectrum_thresholds(const std::vector<int>& table, int nbins);
 std::vector<double> spectrum_k_axis(int N, int mode, int nbins, double L);
 
 }  // namespace qx

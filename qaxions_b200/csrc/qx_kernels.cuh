@@ -348,6 +348,74 @@ __global__ void __launch_bounds__(256, 3) k_x_fwd(XArgs<R> a) {
     }
 }
 
+// Diagnostics of psi and V in one read: per block, part[i * gridDim.x + block] =
+// sum |psi|^2 (i = 0), max |psi|^2 (1), sum V |psi|^2 (2), max |V| (3) and
+// sum over rows and modes of nx^2 |psi^_x|^2 (4), all FP64.  The kinetic energy
+// separates by axis: by Parseval along the other axes, sum k^2 |psi^|^2 over the
+// full transform is the sum over axes of n^2 |F_axis psi|^2 times the other axes'
+// lengths, so it needs one 1D transform per axis that is never stored (three
+// reads of psi) instead of a full transform (two writes and three reads).  512^3
+// FP32 mass and energy 1.74 -> 1.09 ms: 28 bytes per site instead of 60; the y and
+// z shares (346 us each) are bound by their transforms, not by their reads.
+template <int N, typename R>
+__global__ void __launch_bounds__(256, 2) k_x_energy(XArgs<R> a, double* part) {
+    using C = cx_t<R>;
+    constexpr int E = qx_row_efull(N);
+    constexpr bool PAIRED = row_paired<N>();
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    __shared__ double red[256];
+    XTabs<C> tb;
+    C* sm = x_setup<N, R>(a, smem_raw, tb);
+    const int t = threadIdx.x;
+    RowAcc<C> acc{sm, warp_lanes_mask()};
+    double rho = 0.0, rmax = 0.0, vrho = 0.0, vmax = 0.0, kin = 0.0;
+    auto site = [&](const C& p, R v) {
+        const double r = (double)p.x * p.x + (double)p.y * p.y;
+        rho += r;
+        rmax = fmax_nan(rmax, r);
+        vrho += (double)v * r;
+        vmax = fmax_nan(vmax, fabs((double)v));
+    };
+    for (long row = x_row0(); row < a.rows; row += x_row_step()) {
+        acc.sync();  // this slot's previous row is done with the buffer
+        const C* src = a.in + row * N;
+        const R* pot = a.Vin + row * N;
+        C v[E];
+        if constexpr (PAIRED) {
+            C w[E / 2];
+#pragma unroll
+            for (int e = 0; e < E / 2; ++e) {
+                const int q = in_pos<N / 2, E / 2, 0>(e, t);
+                load_pair(src, q, v[row_pair_idx<N>(e, 0)], v[row_pair_idx<N>(e, 1)]);
+                w[e] = reinterpret_cast<const C*>(pot)[q];
+            }
+#pragma unroll
+            for (int e = 0; e < E / 2; ++e) {
+                site(v[row_pair_idx<N>(e, 0)], w[e].x);
+                site(v[row_pair_idx<N>(e, 1)], w[e].y);
+            }
+        } else {
+#pragma unroll
+            for (int e = 0; e < E; ++e) {
+                const int p = in_pos<N, E, 0>(e, t);
+                v[e] = src[p];
+                site(v[e], pot[p]);
+            }
+        }
+        fft_pencil<N, E, -1, PAIRED ? 1 : 0>(v, acc, t, tw_src<true>(tb.N, tb.N_lo));
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+            const int n = signed_mode(out_pos<N, E>(e, t), N);
+            const double x = v[e].x, y = v[e].y;
+            kin = fma((double)(n * n), fma(x, x, y * y), kin);
+        }
+    }
+    const double s[5] = {block_reduce<0>(rho, red), block_reduce<1>(rmax, red), block_reduce<0>(vrho, red),
+                         block_reduce<1>(vmax, red), block_reduce<0>(kin, red)};
+    if (threadIdx.x == 0 && threadIdx.y == 0)
+        for (int i = 0; i < 5; ++i) part[(long)i * gridDim.x + blockIdx.x] = s[i];
+}
+
 // r2c post-processing of one row held in smem (Z[k], k < M) -> packed X row.
 // X[k] = (A + B)/2 - i W_N^k (A - B)/2, A = Z[k], B = conj(Z[M-k]);
 // col 0 = (Re Z0 + Im Z0) + i (Re Z0 - Im Z0) = X[0] + i X[N/2].
@@ -659,7 +727,6 @@ template <typename R> struct SArgs {
     double scale;        // drift: 1/S
     double pois_c;       // Poisson: -1/(dk^2 S) (times 1/|n|^2)
     double pois_g0;      // Poisson multiplier of the k = 0 mode
-    double* partial;     // per-block reduction output (kinetic)
 };
 
 template <typename C> __device__ __forceinline__ int col_pitch(int TX) {
@@ -695,7 +762,7 @@ __global__ void k_y_pass(SArgs<R> s) {
     }
 }
 
-enum LAOp { LA_FWD = 0, LA_INV = 1, LA_DRIFT = 2, LA_POISSON = 3, LA_KIN = 4 };
+enum LAOp { LA_FWD = 0, LA_INV = 1, LA_DRIFT = 2, LA_POISSON = 3 };
 
 // Poisson multiplier of integer |n|^2 (src/field.cxx:250-256,279-285)
 template <typename R> __device__ __forceinline__ R pois_mult(long M2, const SArgs<R>& s);
@@ -765,20 +832,6 @@ __global__ void k_la_pass(SArgs<R> s) {
     const int nx = (s.X == N) ? signed_mode(x, N) : x;  // half arrays: x < N/2
     const int ny = (s.dim == 3) ? signed_mode(y, N) : 0;
     const long mxy = (long)nx * nx + (long)ny * ny;
-    if constexpr (OP == LA_KIN) {
-        double acc_k = 0.0;
-#pragma unroll
-        for (int e = 0; e < E; ++e) {
-            const int nz = signed_mode(out_pos<N, E>(e, t), N);
-            const double m2 = (double)(mxy + (long)nz * nz);
-            acc_k += m2 * ((double)v[e].x * (double)v[e].x + (double)v[e].y * (double)v[e].y);
-        }
-        __shared__ double red[32];
-        const double tot = block_reduce<0>(acc_k, red);
-        if (threadIdx.x == 0 && threadIdx.y == 0 && threadIdx.z == 0)
-            s.partial[blockIdx.x + (long)gridDim.x * blockIdx.y] = tot;
-        return;
-    }
     if constexpr (OP == LA_DRIFT) {
         // exp(-i dt/2 dk^2 |n|^2)/S = A(nx, ny) B(nz), both in FP64 (same
         // arithmetic as the TMA-fed pass, which tabulates B)

@@ -19,7 +19,7 @@ namespace qx {
 
 template <typename K>
 static void set_smem(K kernel, size_t bytes) {
-    if (bytes > 48 * 1024) {
+    if (bytes > 40 * 1024) {  // (48 KB without the attribute, less the kernel's static arrays)
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
         if (e != cudaSuccess) throw std::runtime_error(std::string("smem attribute: ") + cudaGetErrorString(e));
     }
@@ -55,7 +55,7 @@ template <typename R> static XArgs<R> to_x(const typename Ops<R>::XP& a) {
 template <typename R> static SArgs<R> to_s(const typename Ops<R>::SP& a) {
     SArgs<R> s;
     s.a = a.a; s.tw = a.tw; s.tw_lo = a.tw_lo; s.X = a.X; s.dim = a.dim; s.N = a.N; s.phase_fac = a.phase_fac;
-    s.scale = a.scale; s.pois_c = a.pois_c; s.pois_g0 = a.pois_g0; s.partial = a.partial;
+    s.scale = a.scale; s.pois_c = a.pois_c; s.pois_g0 = a.pois_g0;
     return s;
 }
 

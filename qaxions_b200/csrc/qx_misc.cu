@@ -1,5 +1,6 @@
 // qx_misc.cu -- pointwise, reduction, spectrum-binning and initial-condition
 // kernels (sm_100a).  See qx_misc.hpp for the contracts.
+#include <cmath>
 #include <stdexcept>
 #include <string>
 
@@ -89,9 +90,6 @@ __global__ void __launch_bounds__(kRedThreads) k_reduce(int kind, const cx_t<R>*
             a1 = fmax_nan(a1, r);
         } else if (kind == RED_VABS) {
             a1 = fmax_nan(a1, fabs((double)V[i]));
-        } else if (kind == RED_VRHO) {
-            const cx_t<R> p = psi[i];
-            a0 += (double)V[i] * ((double)p.x * p.x + (double)p.y * p.y);
         } else if (kind == RED_RE2) {
             const double r = (double)psi[i].x;
             a0 += r * r;
@@ -117,9 +115,15 @@ __global__ void k_fold(const double* partial, int n, double* out) {
     }
 }
 
-__global__ void k_fold_sum(const double* partial, long n, double* out) {
-    const double s = warp_fold<0>(partial, n);
-    if (threadIdx.x == 0) out[0] = s;
+// The diagnostics' partials (Ops::energy) folded in a fixed order, one warp per
+// quantity: out = {sum |psi|^2, max |psi|^2, sum V |psi|^2, max |V|, the three
+// axes' kinetic sums}.  Launched <<<1, 7 * 32>>>.
+__global__ void k_fold_energy(const double* part, long cap, long n0, long n1, long n2, double* out) {
+    const int w = threadIdx.x >> 5;
+    double v;
+    if (w < 5) v = (w & 1) ? warp_fold<1>(part + w * n0, n0) : warp_fold<0>(part + w * n0, n0);
+    else v = warp_fold<0>(part + w * cap, w == 5 ? n1 : n2);
+    if ((threadIdx.x & 31) == 0) out[w] = v;
 }
 
 // drift factor tables (qx_misc.hpp)
@@ -190,38 +194,53 @@ __global__ void k_poisson_packed(cx_t<R>* vh, int dim, int N, double pc, double 
     }
 }
 
-// deterministic per-warp aggregation of (bin, value, weight) into warp histograms
-__device__ __forceinline__ void spec_agg(int b, double v, int w, double* hP, long long* hC) {
-    const unsigned peers = __match_any_sync(0xffffffffu, b);
-    double s = 0.0;
-    long long cnt = 0;
-#pragma unroll 4
-    for (int l = 0; l < 32; ++l) {
-        const double vl = __shfl_sync(0xffffffffu, v, l);
-        const int wl = __shfl_sync(0xffffffffu, w, l);
-        if ((peers >> l) & 1u) {
-            s += vl;
-            cnt += wl;
-        }
+// Shell of |n|^2 = M: bin b holds T[b] <= M < T[b + 1] (thresholds of the exact host
+// table; [first, end) the binned range), found from a floating-point guess (an
+// approximate square root or logarithm is enough) and corrected against T;
+// -1 outside.
+__device__ __forceinline__ int spec_bin_of(int M, const int* __restrict__ T, int first, int end, int mode, float g,
+                                           int nbins) {
+    if (M < first || M >= end) return -1;
+    float r;
+    if (mode == 2) {
+        r = __log2f((float)M) * g;
+    } else {
+        asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"((float)M));
+        r = mode == 0 ? r + 0.5f : r * g;
     }
-    const int lane = threadIdx.x & 31;
-    if (b >= 0 && lane == __ffs(peers) - 1) {
-        hP[b] += s;
-        hC[b] += cnt;
+    int b = min(max((int)r, 0), nbins - 1);
+    int lo = __ldg(T + b), hi = __ldg(T + b + 1);
+    while (M < lo) {
+        --b;
+        hi = lo;
+        lo = __ldg(T + b);
     }
-    __syncwarp();
+    while (M >= hi) {
+        ++b;
+        hi = __ldg(T + b + 1);
+    }
+    return b;
 }
 
 // Shell binning with the reference's Hermitian weights
 // (src/spectrum/spectrum.cxx:63-155): weight 2 for 0 < kx < N/2, 1 for the
 // kx = 0 and kx = N/2 modes (both unpacked from column 0).  Sums w |X|^2
 // (the 1/S^2 factor is applied by the caller); counts are exact integers.
-template <typename R>
-__global__ void k_spec_bin(const cx_t<R>* vh, int dim, int N, const int* __restrict__ tab, int nbins,
-                           double* part_P, long long* part_c) {
+//
+// A warp takes 32 consecutive elements.  Along a row kx grows, so the bins are
+// sorted and equal bins are adjacent: a segmented warp scan (five shuffle
+// steps, a fixed tree) leaves every run's sum in its last lane, which adds it to
+// the warp's own histogram; runs of different rows are added one row after the
+// other.  Issue-bound (about 200 instructions per 32 elements); all 32 lanes
+// compared with one another took 64 double shuffles per element instead: the
+// spectrum of 512^3 FP32 in 256 bins 4.21 -> 1.21 ms, this kernel 514 us of it.
+template <int N, typename R>
+__global__ void __launch_bounds__(256) k_spec_bin(const cx_t<R>* vh, long rows, int dim, const int* __restrict__ T,
+                                                  int mode, float g, int nbins, double* part_P, long long* part_c) {
     using C = cx_t<R>;
+    constexpr int X = N / 2;
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    const int nw = blockDim.x >> 5, warp = threadIdx.x >> 5;
+    const int nw = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     double* hPall = reinterpret_cast<double*>(smem_raw);
     long long* hCall = reinterpret_cast<long long*>(hPall + nw * nbins);
     for (int i = threadIdx.x; i < nw * nbins; i += blockDim.x) {
@@ -231,42 +250,82 @@ __global__ void k_spec_bin(const cx_t<R>* vh, int dim, int N, const int* __restr
     __syncthreads();
     double* hP = hPall + warp * nbins;
     long long* hC = hCall + warp * nbins;
-    const int X = N / 2;
-    const long total = (dim == 3 ? (long)N * N : (long)N) * X;
-    const long stride = (long)gridDim.x * blockDim.x;
-    const long iters = (total + stride - 1) / stride;
-    for (long it = 0; it < iters; ++it) {
-        const long i = it * stride + blockIdx.x * (long)blockDim.x + threadIdx.x;
-        int b1 = -1, b2 = -1, w1 = 0, w2 = 0;
-        double v1 = 0.0, v2 = 0.0;
-        if (i < total) {
-            const int x = (int)(i % X);
-            const long rest = i / X;
-            const int y = dim == 3 ? (int)(rest % N) : (int)rest;
-            const int z = dim == 3 ? (int)(rest / N) : 0;
-            const long ny = signed_mode(y, N), nz = dim == 3 ? signed_mode(z, N) : 0;
-            const C c = vh[i];
-            if (x > 0) {
-                b1 = tab[(long)x * x + ny * ny + nz * nz];
-                w1 = 2;
-                v1 = 2.0 * ((double)c.x * c.x + (double)c.y * c.y);
-            } else {
-                const C cm = vh[mirror0(i, dim, N)];
-                const double ax = 0.5 * ((double)c.x + cm.x), ay = 0.5 * ((double)c.y - cm.y);
-                const double bx = 0.5 * ((double)c.x - cm.x), by = 0.5 * ((double)c.y + cm.y);
-                const long mA = ny * ny + nz * nz;
-                b1 = tab[mA];
-                w1 = 1;
-                v1 = ax * ax + ay * ay;
-                b2 = tab[mA + (long)X * X];
-                w2 = 1;
-                v2 = bx * bx + by * by;
+    const int first = __ldg(T), end = __ldg(T + nbins);
+    const int total = (int)(rows * X);  // at most 2^26
+    const int units = (total + 31) / 32;
+    constexpr int U = 4;  // units in flight together
+    const int ustep = gridDim.x * nw;
+    for (int u0 = blockIdx.x * nw + warp; u0 < units; u0 += U * ustep) {
+        C c[U], cm[U];
+#pragma unroll
+        for (int j = 0; j < U; ++j) {
+            const int i = (u0 + j * ustep) * 32 + lane;
+            c[j] = mk<C>(0, 0);
+            cm[j] = c[j];
+            if (i < total) {
+                c[j] = vh[i];
+                if (i % X == 0) cm[j] = vh[mirror0(i, dim, N)];
             }
-            if (b1 < 0) w1 = 0;
-            if (b2 < 0) w2 = 0;
         }
-        spec_agg(b1, v1, w1, hP, hC);
-        spec_agg(b2, v2, w2, hP, hC);
+        double v[U], v2[U];
+        int b[U], b2[U], row[U];
+        unsigned heads[U];
+#pragma unroll
+        for (int j = 0; j < U; ++j) {
+            const int i = (u0 + j * ustep) * 32 + lane;
+            const bool in = i < total;
+            const int x = i % X;
+            row[j] = i / X;
+            const int y = dim == 3 ? row[j] % N : row[j], z = dim == 3 ? row[j] / N : 0;
+            const int ny = signed_mode(y, N), nz = dim == 3 ? signed_mode(z, N) : 0;
+            const int m0 = ny * ny + nz * nz;
+            v2[j] = 0.0;
+            b2[j] = -1;
+            if (x > 0) {
+                v[j] = 2.0 * ((double)c[j].x * c[j].x + (double)c[j].y * c[j].y);
+            } else {
+                const double ax = 0.5 * ((double)c[j].x + cm[j].x), ay = 0.5 * ((double)c[j].y - cm[j].y);
+                const double bx = 0.5 * ((double)c[j].x - cm[j].x), by = 0.5 * ((double)c[j].y + cm[j].y);
+                v[j] = ax * ax + ay * ay;
+                if (in) b2[j] = spec_bin_of(m0 + X * X, T, first, end, mode, g, nbins);
+                v2[j] = bx * bx + by * by;
+            }
+            b[j] = in ? spec_bin_of(m0 + x * x, T, first, end, mode, g, nbins) : -1;
+            const int bp = __shfl_up_sync(0xffffffffu, b[j], 1);
+            heads[j] = __ballot_sync(0xffffffffu, lane == 0 || x == 0 || b[j] != bp);
+        }
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+#pragma unroll
+            for (int j = 0; j < U; ++j) {
+                const int start = 31 - __clz(heads[j] & (0xffffffffu >> (31 - lane)));
+                const double t = __shfl_up_sync(0xffffffffu, v[j], d);
+                if (lane - d >= start) v[j] += t;
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < U; ++j) {
+            const int start = 31 - __clz(heads[j] & (0xffffffffu >> (31 - lane)));
+            const bool tail = (lane == 31 || ((heads[j] >> (lane + 1)) & 1u)) && b[j] >= 0;
+            // kx of the run's first element (weight 1 when 0)
+            const int xs = ((u0 + j * ustep) * 32 + start) % X;
+            const long long cnt = 2 * (lane - start + 1) - (xs == 0 ? 1 : 0);
+            // rows of this unit, one after the other
+            const int ph = X % 32 == 0 ? 0 : row[j] - __shfl_sync(0xffffffffu, row[j], 0);
+            const int nph = X % 32 == 0 ? 1 : __shfl_sync(0xffffffffu, ph, 31) + 1;
+            for (int p = 0; p < nph; ++p) {
+                if (tail && ph == p) {
+                    hP[b[j]] += v[j];
+                    hC[b[j]] += cnt;
+                }
+                __syncwarp();
+                if (b2[j] >= 0 && ph == p) {
+                    hP[b2[j]] += v2[j];
+                    hC[b2[j]] += 1;
+                }
+                __syncwarp();
+            }
+        }
     }
     __syncthreads();
     for (int b = threadIdx.x; b < nbins; b += blockDim.x) {
@@ -281,15 +340,24 @@ __global__ void k_spec_bin(const cx_t<R>* vh, int dim, int N, const int* __restr
     }
 }
 
+// one warp per bin folds the blocks' partials in a fixed order
 __global__ void k_spec_fold(const double* part_P, const long long* part_c, int nblk, int nbins, double* P,
                             long long* cnt) {
-    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < nbins; b += gridDim.x * blockDim.x) {
-        double s = 0.0;
-        long long c = 0;
-        for (int k = 0; k < nblk; ++k) {
-            s += part_P[(long)k * nbins + b];
-            c += part_c[(long)k * nbins + b];
-        }
+    const int lane = threadIdx.x & 31;
+    const int b = (int)((blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5);
+    if (b >= nbins) return;
+    double s = 0.0;
+    long long c = 0;
+    for (int k = lane; k < nblk; k += 32) {
+        s += part_P[(long)k * nbins + b];
+        c += part_c[(long)k * nbins + b];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        s += __shfl_xor_sync(0xffffffffu, s, o);
+        c += __shfl_xor_sync(0xffffffffu, c, o);
+    }
+    if (lane == 0) {
         P[b] = s;
         cnt[b] = c;
     }
@@ -316,9 +384,8 @@ void Misc<R>::reduce(int kind, const C* psi, const R* V, long S, double* partial
     k_fold<<<1, 32, 0, st>>>(partial, kRedBlocks, out);
     QX_CHECK_LAUNCH();
 }
-template <typename R>
-void Misc<R>::fold_sum(const double* partial, long n, double* out, cudaStream_t st) {
-    k_fold_sum<<<1, 32, 0, st>>>(partial, n, out);
+void fold_energy(const double* part, long cap, const long (&n)[3], double* out, cudaStream_t st) {
+    k_fold_energy<<<1, 7 * 32, 0, st>>>(part, cap, n[0], n[1], n[2], out);
     QX_CHECK_LAUNCH();
 }
 template <typename R>
@@ -327,23 +394,46 @@ void Misc<R>::poisson_packed(C* vh, int dim, int N, double pc, double g0, cudaSt
     k_poisson_packed<R><<<grid_for(total, 256), 256, 0, st>>>(vh, dim, N, pc, g0);
     QX_CHECK_LAUNCH();
 }
-template <typename R>
-int Misc<R>::spectrum_bin(const C* vh, int dim, int N, const int* tab, int nbins, double* part_P,
-                          long long* part_c, cudaStream_t st) {
-    const int threads = 256, nblk = 296;
+template <int N, typename R>
+static void launch_spec_bin(const cx_t<R>* vh, long rows, int dim, const int* T, int mode, int nbins, int nblk,
+                            double* part_P, long long* part_c, cudaStream_t st) {
+    const int threads = 256;
     const size_t smem = (size_t)(threads / 32) * nbins * (sizeof(double) + sizeof(long long));
     if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(k_spec_bin<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = cudaFuncSetAttribute(k_spec_bin<N, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) throw std::runtime_error(std::string("smem attribute: ") + cudaGetErrorString(e));
     }
-    k_spec_bin<R><<<nblk, threads, smem, st>>>(vh, dim, N, tab, nbins, part_P, part_c);
+    // the guess of spec_bin_of: shells sqrt(M), nbins sqrt(M) / nmax, nbins log(M) / (2 log(nmax))
+    const float nmax = (float)(N / 2);
+    const float g = mode == 0 ? 1.0f : mode == 1 ? (float)nbins / nmax : (float)nbins / (2.0f * std::log2(nmax));
+    k_spec_bin<N, R><<<nblk, threads, smem, st>>>(vh, rows, dim, T, mode, g, nbins, part_P, part_c);
     QX_CHECK_LAUNCH();
+}
+template <typename R>
+int Misc<R>::spectrum_bin(const C* vh, int dim, int N, const int* T, int mode, int nbins, double* part_P,
+                          long long* part_c, cudaStream_t st) {
+    const long rows = dim == 3 ? (long)N * N : N;
+    // 6 blocks per SM, fewer where a warp would get no four units of 32 elements
+    const long want = (rows * (N / 2) + 1023) / 1024;
+    const int nblk = (int)(want < 1 ? 1 : want > kSpecBlocks ? kSpecBlocks : want);
+    switch (N) {
+        case 4: launch_spec_bin<4, R>(vh, rows, dim, T, mode, nbins, nblk, part_P, part_c, st); break;
+        case 8: launch_spec_bin<8, R>(vh, rows, dim, T, mode, nbins, nblk, part_P, part_c, st); break;
+        case 16: launch_spec_bin<16, R>(vh, rows, dim, T, mode, nbins, nblk, part_P, part_c, st); break;
+        case 32: launch_spec_bin<32, R>(vh, rows, dim, T, mode, nbins, nblk, part_P, part_c, st); break;
+        case 64: launch_spec_bin<64, R>(vh, rows, dim, T, mode, nbins, nblk, part_P, part_c, st); break;
+        case 96: launch_spec_bin<96, R>(vh, rows, dim, T, mode, nbins, nblk, part_P, part_c, st); break;
+        case 128: launch_spec_bin<128, R>(vh, rows, dim, T, mode, nbins, nblk, part_P, part_c, st); break;
+        case 256: launch_spec_bin<256, R>(vh, rows, dim, T, mode, nbins, nblk, part_P, part_c, st); break;
+        case 512: launch_spec_bin<512, R>(vh, rows, dim, T, mode, nbins, nblk, part_P, part_c, st); break;
+        default: throw std::invalid_argument("unsupported grid size N=" + std::to_string(N));
+    }
     return nblk;
 }
 template <typename R>
 void Misc<R>::spectrum_fold(const double* part_P, const long long* part_c, int nblk, int nbins, double* P,
                             long long* cnt, cudaStream_t st) {
-    k_spec_fold<<<(nbins + 127) / 128, 128, 0, st>>>(part_P, part_c, nblk, nbins, P, cnt);
+    k_spec_fold<<<(nbins + 3) / 4, 128, 0, st>>>(part_P, part_c, nblk, nbins, P, cnt);
     QX_CHECK_LAUNCH();
 }
 template <typename R>

@@ -14,10 +14,11 @@ namespace qx {
 constexpr int kRedBlocks = 592;   // 4 x 148 SMs: per-block partials of reductions
 constexpr int kRedThreads = 256;
 
+constexpr int kSpecBlocks = 888;  // 6 x 148 SMs: most blocks of the shell binning
+
 enum RedKind {
     RED_RHO = 0,      // out[0] = sum |psi|^2, out[1] = max |psi|^2
     RED_VABS = 1,     // out[0] = max |V|
-    RED_VRHO = 2,     // out[0] = sum V |psi|^2
     RED_RE2 = 3,      // out[0] = sum (Re psi)^2  (GRF normalisation)
     RED_RE = 4,       // out[0] = sum Re psi        (IC density mean)
 };
@@ -30,14 +31,14 @@ template <typename R> struct Misc {
     static void rho_to_V(const C* psi, R* V, long S, cudaStream_t st);
     // reductions; partial must hold 2*kRedBlocks doubles, out 2 doubles
     static void reduce(int kind, const C* psi, const R* V, long S, double* partial, double* out, cudaStream_t st);
-    // fold n per-block sums in order: out[0] = sum partial[0..n)
-    static void fold_sum(const double* partial, long n, double* out, cudaStream_t st);
     // Poisson multiplier on a fully transformed packed half spectrum
     // (Field::Poisson, src/field.cxx:230-291)
     static void poisson_packed(C* vh, int dim, int N, double pois_c, double pois_g0, cudaStream_t st);
-    // shell binning of a fully transformed packed half spectrum; part_P and
-    // part_c hold nblk*nbins entries; returns nblk (the fold size)
-    static int spectrum_bin(const C* vh, int dim, int N, const int* bin_of_m2, int nbins, double* part_P,
+    // shell binning of a fully transformed packed half spectrum.  T: the shells'
+    // thresholds in |n|^2 (spectrum_thresholds); mode as in spectrum_bin_table;
+    // part_P and part_c hold nblk*nbins entries, nblk <= kSpecBlocks returned (the
+    // fold size)
+    static int spectrum_bin(const C* vh, int dim, int N, const int* T, int mode, int nbins, double* part_P,
                             long long* part_c, cudaStream_t st);
     static void spectrum_fold(const double* part_P, const long long* part_c, int nblk, int nbins, double* P,
                               long long* cnt, cudaStream_t st);
@@ -48,6 +49,11 @@ template <typename R> struct Misc {
     static void real_to_f64(const R* src, double* dst, long n, cudaStream_t st);
     static void scale(C* psi, double s, long n, cudaStream_t st);
 };
+
+// fold the partials of Ops::energy (cap = its energy_blocks(), n its block counts):
+// out[0..6] = sum |psi|^2, max |psi|^2, sum V |psi|^2, max |V|, and the x, y, z
+// sums of n^2 |F_axis psi|^2
+void fold_energy(const double* part, long cap, const long (&n)[3], double* out, cudaStream_t st);
 
 // drift factor tables of exp(i fac |n|^2) / S = A(nx, ny) B(nz) (FP64,
 // arguments reduced mod 2 pi): A = exp(i fac (nx^2 + ny^2)) at t[y * N + x]

@@ -62,9 +62,14 @@ template <typename R> struct Ops {
     static void x_c2r(int N, const XP& a, int flags, const Tune& tu, cudaStream_t st);
     // y pass of an [outer][N][X] array (3D only)
     static void y_pass(int N, int outer, const SP& s, int sign, const Tune& tu, cudaStream_t st);
-    // last-axis pass; returns the number of blocks (partials written for OP_KIN)
-    static long la_pass(int N, const SP& s, int op, const Tune& tu, cudaStream_t st);
-    static long la_blocks(int N, int X, int dim, int op, const Tune& tu);
+    // last-axis pass
+    static void la_pass(int N, const SP& s, int op, const Tune& tu, cudaStream_t st);
+    // Diagnostics of psi (a.in, s.a) and V (a.Vin), one read of psi per axis
+    // (k_x_energy): per-block partials in part (7 * energy_blocks() doubles):
+    // five arrays of n[0] from the x rows back to back, then at 5 and 6 *
+    // energy_blocks() the n[1] y and n[2] z shares of sum n^2 |F_axis psi|^2
+    static void energy(int N, const XP& a, const SP& s, double* part, long (&n)[3], const Tune& tu, cudaStream_t st);
+    static long energy_blocks();
     // The drift chain (y forward, z forward + drift + z inverse, y inverse) of a
     // 3D wave-function array as one kernel over x-slabs of sw 8-column tiles
     // (FP32, N >= 16, sw = 1 or 2).  chain_slabs: slabs of the array (0: the

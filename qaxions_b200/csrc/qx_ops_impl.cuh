@@ -66,8 +66,8 @@ static int sm_count() {
     return cache[dev];
 }
 
-template <typename R, int NN, typename K>
-static void launch_x(K kernel, const XArgs<R>& x, int P, cudaStream_t st, int stage_elems = 0) {
+template <typename R, int NN, typename K, typename... A>
+static long launch_x(K kernel, const XArgs<R>& x, int P, cudaStream_t st, int stage_elems = 0, A... args) {
     using C = cx_t<R>;
     const int T = qx_row_threads(NN);
     // tables + P row buffers (+ P staging buffers and alignment slack)
@@ -94,8 +94,9 @@ static void launch_x(K kernel, const XArgs<R>& x, int P, cudaStream_t st, int st
     long grid = (long)sm_count() * bps;
     if (grid > blocks) grid = blocks;
     dim3 blk(T, P);
-    kernel<<<(unsigned)grid, blk, smem, st>>>(x);
+    kernel<<<(unsigned)grid, blk, smem, st>>>(x, args...);
     QX_LAUNCH_CHECK();
+    return grid;
 }
 
 template <typename R>
@@ -469,8 +470,8 @@ void Ops<R>::y_pass(int N, int outer, const SP& a, int sign, const Tune& tu, cud
     });
 }
 
-// direct-load last-axis kernel of an op; the FP32 drift and kinetic passes
-// always take double-float twiddles, the Poisson pass never, the plain
+// direct-load last-axis kernel of an op; the FP32 drift pass always takes
+// double-float twiddles, the Poisson pass never, the plain
 // transforms when `df` (a wave-function array)
 template <int NN, typename R>
 static void (*la_kernel(int op, bool df))(SArgs<R>) {
@@ -480,7 +481,6 @@ static void (*la_kernel(int op, bool df))(SArgs<R>) {
         case OP_INV: return df ? k_la_pass<NN, R, LA_INV, f32> : k_la_pass<NN, R, LA_INV, false>;
         case OP_DRIFT: return k_la_pass<NN, R, LA_DRIFT, f32>;
         case OP_POISSON: return k_la_pass<NN, R, LA_POISSON, false>;
-        case OP_KIN: return k_la_pass<NN, R, LA_KIN, f32>;
     }
     throw std::invalid_argument("la_pass: bad op");
 }
@@ -494,18 +494,28 @@ static int la_max_threads(int op, bool df) {
 }
 
 template <typename R>
-long Ops<R>::la_blocks(int N, int X, int dim, int op, const Tune& tu) {
-    using C = cx_t<R>;
-    if (tu.tma) return (long)sm_count() * 32;  // upper bound of the persistent grid
+long Ops<R>::energy_blocks() { return (long)sm_count() * 32; }
+
+template <typename R>
+void Ops<R>::energy(int N, const XP& a, const SP& s, double* part, long (&n)[3], const Tune& tu, cudaStream_t st) {
+    const XArgs<R> x = to_x<R>(a);
+    SP p = s;
+    const long cap = energy_blocks();
+    const int nb = s.batch > 0 ? s.batch : 1;
+    const int P = x_rows_per_block(N, a.rows, tu.x_rows);
     QX_FOR_N(N, {
-        constexpr int E = qx_col_e(NN);
-        const int T = NN / E;
-        const int G = (dim == 3 && op == OP_POISSON) ? 2 : 1;
-        const int tx = pick_tx(X, T, G, tu.la_tx, sizeof(C), NN, la_max_threads<NN, R>(op, X == NN));
-        const long gy = dim == 3 ? (G == 2 ? NN / 2 : NN) : 1;
-        return (long)(X / tx) * gy;
+        n[0] = launch_x<R, NN>(k_x_energy<NN, R>, x, P, st, 0, part);
+        const bool d3 = s.dim == 3;
+        const int planes = d3 ? nb * NN : nb;  // y pencils: one plane per tile row
+        p.partial = part + 5 * cap;
+        n[1] = launch_tma<NN, R, OP_KIN>(p, planes, planes, 1, 0, 0, tu, st);
+        n[2] = 0;
+        if (d3) {
+            p.partial = part + 6 * cap;
+            n[2] = launch_tma<NN, R, OP_KIN>(p, planes, planes, 2, 1, 0, tu, st);
+        }
     });
-    return 0;
+    if (n[0] > cap || n[1] > cap || n[2] > cap) throw std::logic_error("energy: more blocks than partials");
 }
 
 template <int NN, typename R>
@@ -526,7 +536,7 @@ static void launch_col0(const typename Ops<R>::SP& a, cudaStream_t st) {
 }
 
 template <typename R>
-long Ops<R>::la_pass(int N, const SP& a, int op, const Tune& tu, cudaStream_t st) {
+void Ops<R>::la_pass(int N, const SP& a, int op, const Tune& tu, cudaStream_t st) {
     using C = cx_t<R>;
     const SArgs<R> s = to_s<R>(a);
     const bool df = sizeof(R) == 4 && a.tw_lo != nullptr;
@@ -535,20 +545,18 @@ long Ops<R>::la_pass(int N, const SP& a, int op, const Tune& tu, cudaStream_t st
             const int d3 = a.dim == 3 ? 1 : 0;
             const int nb = a.batch > 0 ? a.batch : 1;
             const int NZ = d3 ? nb * NN : nb, outer = d3 ? nb * NN : nb, pdim = d3 ? 2 : 1;
-            long grid = 0;
             switch (op) {
-                case OP_FWD: grid = launch_tma<NN, R, OP_FWD>(a, NZ, outer, pdim, d3, 0, tu, st); break;
-                case OP_INV: grid = launch_tma<NN, R, OP_INV>(a, NZ, outer, pdim, d3, 0, tu, st); break;
-                case OP_DRIFT: grid = launch_tma<NN, R, OP_DRIFT>(a, NZ, outer, pdim, d3, 0, tu, st); break;
+                case OP_FWD: launch_tma<NN, R, OP_FWD>(a, NZ, outer, pdim, d3, 0, tu, st); break;
+                case OP_INV: launch_tma<NN, R, OP_INV>(a, NZ, outer, pdim, d3, 0, tu, st); break;
+                case OP_DRIFT: launch_tma<NN, R, OP_DRIFT>(a, NZ, outer, pdim, d3, 0, tu, st); break;
                 case OP_POISSON:
-                    grid = launch_tma<NN, R, OP_POISSON>(a, NZ, outer, pdim, d3, d3, tu, st);
+                    launch_tma<NN, R, OP_POISSON>(a, NZ, outer, pdim, d3, d3, tu, st);
                     if (d3) launch_col0<NN, R>(a, st);
                     break;
-                case OP_KIN: grid = launch_tma<NN, R, OP_KIN>(a, NZ, outer, pdim, d3, 0, tu, st); break;
                 default: throw std::invalid_argument("la_pass: bad op");
             }
-            return grid;
         });
+        return;
     }
     if (a.batch > 1) throw std::invalid_argument("batched arrays need the TMA-fed strided passes");
     QX_FOR_N(N, {
@@ -564,9 +572,7 @@ long Ops<R>::la_pass(int N, const SP& a, int op, const Tune& tu, cudaStream_t st
         set_smem(kern, smem);
         kern<<<grd, blk, smem, st>>>(s);
         QX_LAUNCH_CHECK();
-        return (long)grd.x * grd.y;
     });
-    return 0;
 }
 
 // ---------------------------------------------------------------------------

@@ -314,15 +314,17 @@ __global__ void __launch_bounds__((tma_block_threads<N, R, PW, TXF>()), (tma_blo
         };
         bool store = true;
         if constexpr (OP == OP_KIN) {
+            // this axis' share of the kinetic energy (k_x_energy)
 #pragma unroll
-            for (int h = 0; h < PW; ++h) {
-                const long mxy = mxy_of(h);
+            for (int e = 0; e < E; ++e) {
+                const int n = signed_mode(out_pos<NL, E>(e, t), N);
+                double p = 0.0;
 #pragma unroll
-                for (int e = 0; e < E; ++e) {
-                    const int nz = signed_mode(out_pos<NL, E>(e, t), N);
+                for (int h = 0; h < PW; ++h) {
                     const C u = pen(v[e], h);
-                    kin += (double)(mxy + (long)nz * nz) * ((double)u.x * (double)u.x + (double)u.y * (double)u.y);
+                    p = fma((double)u.x, (double)u.x, fma((double)u.y, (double)u.y, p));
                 }
+                kin = fma((double)(n * n), p, kin);
             }
             store = false;
         } else if constexpr (OP == OP_DRIFT || OP == OP_POISSON) {
@@ -624,15 +626,17 @@ __global__ void __launch_bounds__(kWpThreads * WPP, 1) k_pencil_wp(const __grid_
         };
         bool store = true;
         if constexpr (OP == OP_KIN) {
+            // this axis' share of the kinetic energy (k_x_energy)
 #pragma unroll
-            for (int h = 0; h < PW; ++h) {
-                const long mxy = mxy_of(h);
+            for (int e = 0; e < E; ++e) {
+                const int n = signed_mode(out_pos<NL, E>(e, t), N);
+                double p = 0.0;
 #pragma unroll
-                for (int e = 0; e < E; ++e) {
-                    const int nz = signed_mode(out_pos<NL, E>(e, t), N);
+                for (int h = 0; h < PW; ++h) {
                     const C u = pen(v[e], h);
-                    kin += (double)(mxy + (long)nz * nz) * ((double)u.x * (double)u.x + (double)u.y * (double)u.y);
+                    p = fma((double)u.x, (double)u.x, fma((double)u.y, (double)u.y, p));
                 }
+                kin = fma((double)(n * n), p, kin);
             }
             store = false;
         } else if constexpr (OP == OP_DRIFT || OP == OP_POISSON) {
