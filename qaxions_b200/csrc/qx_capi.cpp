@@ -700,6 +700,8 @@ void ens_check_flag(qx_ens_s& e) {
     }
 }
 
+constexpr int kEnsGraphBodies = 8;  // steps of every group per replay (per-size launches)
+
 void ens_capture(qx_ens_s& e) {
     if (e.exec) cudaGraphExecDestroy(e.exec);
     e.exec = nullptr;
@@ -721,7 +723,8 @@ void ens_capture(qx_ens_s& e) {
             ens_enqueue_mixed(e, d);
         } else {
             ens_fork(e);  // the group streams join the capture
-            for (auto& g : e.groups) g->enqueue_body(false);
+            for (int i = 0; i < kEnsGraphBodies; ++i)
+                for (auto& g : e.groups) g->enqueue_body(false);
             ens_join(e);
         }
     } catch (...) {
@@ -737,9 +740,12 @@ void ens_capture(qx_ens_s& e) {
     for (auto& g : e.groups) e.exec_dt.push_back(g->dt());
 }
 
-// the merged loop of every box: prologues and the first and last bodies run
-// eagerly on the group streams; the bodies in between are one graph replay
-// per step over all groups
+// the merged loop of every box: prologues and the last bodies run eagerly on the
+// group streams.  The bodies in between are graph replays over all groups:
+// kEnsGraphBodies steps of every group per replay (a branch per group, joined once
+// per replay, so a fast group does not wait for a slow one at every step), or
+// one step per replay in the mixed-size modes; what is left, and calls too
+// short to pay for a capture, run eagerly.
 void ens_step(qx_ens_s& e, int nsteps) {
     if (nsteps <= 0) return;
     if (!e.s0) {
@@ -751,15 +757,19 @@ void ens_step(qx_ens_s& e, int nsteps) {
     for (auto& g : e.groups) g->step_begin();
     if (nsteps > 1) {
         for (auto& g : e.groups) g->enqueue_body(false);  // eager (also sets kernel attributes)
-        if (nsteps > 2) {
-            bool same = e.exec && e.exec_dt.size() == e.groups.size();
-            for (size_t i = 0; same && i < e.groups.size(); ++i) same = e.exec_dt[i] == e.groups[i]->dt();
+        int left = nsteps - 2;
+        const int per = e.mixed ? 1 : kEnsGraphBodies;
+        bool same = e.exec && e.exec_dt.size() == e.groups.size();
+        for (size_t i = 0; same && i < e.groups.size(); ++i) same = e.exec_dt[i] == e.groups[i]->dt();
+        if (left >= (same || e.mixed ? per : 2 * per)) {
             if (!same) ens_capture(e);
             for (auto& g : e.groups) g->prepare_replay();
             ens_join(e);
-            for (int i = 0; i < nsteps - 2; ++i) QX_CU(cudaGraphLaunch(e.exec, e.s0));
+            for (; left >= per; left -= per) QX_CU(cudaGraphLaunch(e.exec, e.s0));
             ens_fork(e);
         }
+        for (; left > 0; --left)
+            for (auto& g : e.groups) g->enqueue_body(false);
     }
     for (auto& g : e.groups) g->enqueue_body(true);
     for (auto& g : e.groups) g->step_end(nsteps);

@@ -42,17 +42,6 @@ void Ops<R>::stage_twiddles(const C* nat, int L, C* out) {
 }
 
 
-// rows per block for x passes: T*P ~ 256 threads, P | rows
-static int x_rows_per_block(int N, long rows, int want) {
-    QX_FOR_N(N, {
-        const int T = qx_row_threads(NN);
-        int P = want > 0 ? want : (256 / T > 0 ? 256 / T : 1);
-        while (P > 1 && (rows % P)) P >>= 1;
-        return P;
-    });
-    return 1;
-}
-
 static int sm_count() {
     static int cache[64] = {0};
     int dev = 0;
@@ -64,6 +53,20 @@ static int sm_count() {
         cache[dev] = n > 0 ? n : 1;
     }
     return cache[dev];
+}
+
+// rows per block for x passes: T*P ~ 256 threads, P | rows
+static int x_rows_per_block(int N, long rows, int want) {
+    QX_FOR_N(N, {
+        const int T = qx_row_threads(NN);
+        int P = want > 0 ? want : (256 / T > 0 ? 256 / T : 1);
+        while (P > 1 && (rows % P)) P >>= 1;
+        // few rows: smaller blocks, down to one warp, until they cover the SMs
+        if (want == 0)
+            while (P > 1 && P % 2 == 0 && T * (P / 2) % 32 == 0 && rows / P < sm_count()) P >>= 1;
+        return P;
+    });
+    return 1;
 }
 
 template <typename R, int NN, typename K, typename... A>
@@ -94,8 +97,7 @@ static long launch_x(K kernel, const XArgs<R>& x, int P, cudaStream_t st, int st
     long grid = (long)sm_count() * bps;
     if (grid > blocks) grid = blocks;
     dim3 blk(T, P);
-    kernel<<<(unsigned)grid, blk, smem, st>>>(x, args...);
-    QX_LAUNCH_CHECK();
+    launch_dep(kernel, dim3((unsigned)grid), blk, smem, st, x, args...);
     return grid;
 }
 
@@ -319,8 +321,7 @@ static long launch_tma_e(const typename Ops<R>::SP& a, int NZ, int outer, int pe
     long grid = (long)sm_count() * bps;
     if (grid > s.n_tiles) grid = s.n_tiles;
     dim3 blk(SWZ ? g.TX / PW / 2 : g.TX / PW, g.T, SWZ ? 2 : 1);
-    kern<<<(unsigned)grid, blk, smem, st>>>(tm, s);
-    QX_LAUNCH_CHECK();
+    launch_dep(kern, dim3((unsigned)grid), blk, smem, st, tm, s);
     return grid;
 }
 
@@ -362,8 +363,7 @@ static long launch_wp(const typename Ops<R>::SP& a, int NZ, int outer, int penci
         set_smem(kern, smem);
         long grid = (long)sm_count();
         if (grid > s.n_tiles) grid = s.n_tiles;
-        kern<<<(unsigned)grid, dim3(kWpThreads * WPP), smem, st>>>(tm, s);
-        QX_LAUNCH_CHECK();
+        launch_dep(kern, dim3((unsigned)grid), dim3(kWpThreads * WPP), smem, st, tm, s);
         return grid;
     } else {
         (void)a, (void)NZ, (void)outer, (void)pencil_dim, (void)la3d, (void)col0_ext, (void)st;
@@ -526,13 +526,11 @@ static void launch_col0(const typename Ops<R>::SP& a, cudaStream_t st) {
     dim3 grd(NN / 2, a.batch > 0 ? a.batch : 1);
     if constexpr (strided_plan1<NN>()) {
         if (a.plan == 1) {
-            k_poisson_col0<NN, R, 1><<<grd, blk, 2 * NN * sizeof(C), st>>>(a.a, a.tw, a.tw_lo, a.pois_c, a.pois_g0);
-            QX_LAUNCH_CHECK();
+            launch_dep(k_poisson_col0<NN, R, 1>, grd, blk, 2 * NN * sizeof(C), st, a.a, a.tw, a.tw_lo, a.pois_c, a.pois_g0);
             return;
         }
     }
-    k_poisson_col0<NN, R><<<grd, blk, 2 * NN * sizeof(C), st>>>(a.a, a.tw, a.tw_lo, a.pois_c, a.pois_g0);
-    QX_LAUNCH_CHECK();
+    launch_dep(k_poisson_col0<NN, R>, grd, blk, 2 * NN * sizeof(C), st, a.a, a.tw, a.tw_lo, a.pois_c, a.pois_g0);
 }
 
 template <typename R>

@@ -31,7 +31,7 @@ template <int NN, typename R, typename K>
 static void launch_plane(K kern, const XArgs<R>& x, cudaStream_t st) {
     using G = PlaneGeo<NN, R>;
     set_smem(kern, G::SMEM);
-    launch_pdl(kern, dim3((unsigned)(x.rows / NN)), dim3(G::TB), G::SMEM, st, x);
+    launch_dep(kern, dim3((unsigned)(x.rows / NN)), dim3(G::TB), G::SMEM, st, x);
 }
 
 template <typename R> void Plane<R>::inv(int N, const XP& a, bool r2c, cudaStream_t st) {
@@ -88,12 +88,12 @@ static void launch_col(const typename Ops<R>::SP& a, int op, cudaStream_t st) {
         auto kern = k_col<NN, R, OP_DRIFT, UX, D3>;
         const size_t smem = G::smem(OP_DRIFT, D3);
         set_smem(kern, smem);
-        launch_pdl(kern, dim3(grid), dim3(G::NT), smem, st, s, a.axy);
+        launch_dep(kern, dim3(grid), dim3(G::NT), smem, st, s, a.axy);
     } else {
         auto kern = k_col<NN, R, OP_POISSON, UX, D3>;
         const size_t smem = G::smem(OP_POISSON, D3);
         set_smem(kern, smem);
-        launch_pdl(kern, dim3(grid), dim3(G::NT + (D3 ? G::TX : 0)), smem, st, s, (const double2*)nullptr);
+        launch_dep(kern, dim3(grid), dim3(G::NT + (D3 ? G::TX : 0)), smem, st, s, (const double2*)nullptr);
     }
 }
 

@@ -251,6 +251,13 @@ __global__ void __launch_bounds__((tma_block_threads<N, R, PW, TXF>()), (tma_blo
         tws[i] = s.tw[i];
         if constexpr (DF) tws_lo[i] = s.tw_lo[i];
     }
+    if (tid == 0) {
+        s_abort = 0;
+        for (int b = 0; b < s.nbuf; ++b) mbar_init(smem_u32(&mbar[b]), 1);
+        fence_mbar_init();
+    }
+    // (the drift tables and the state are earlier kernels')
+    pdl_wait();
     if constexpr (OP == OP_DRIFT) {
         const double2* gbz = s.axy + (s.la3d ? (long)N * N : (long)N);
         for (int i = tid; i < N; i += nthr) bz[i] = gbz[i];
@@ -258,9 +265,6 @@ __global__ void __launch_bounds__((tma_block_threads<N, R, PW, TXF>()), (tma_blo
             for (int j = tid; j < TX; j += nthr) aslot[j] = *a_of_tile(blockIdx.x, j);
     }
     if (tid == 0) {
-        s_abort = 0;
-        for (int b = 0; b < s.nbuf; ++b) mbar_init(smem_u32(&mbar[b]), 1);
-        fence_mbar_init();
         for (int k = 0; k < s.nbuf - 1; ++k) {
             const long id = blockIdx.x + (long)k * gridDim.x;
             if (id < s.n_tiles) issue_load(id, k);
@@ -448,6 +452,7 @@ __global__ void __launch_bounds__((tma_block_threads<N, R, PW, TXF>()), (tma_blo
         }
         return;
     }
+    pdl_launch();
     if (tid == 0) bulk_wait_all();
     if constexpr (OP == OP_KIN) {
         const double tot = block_reduce<0>(kin, red);
@@ -571,15 +576,18 @@ __global__ void __launch_bounds__(kWpThreads * WPP, 1) k_pencil_wp(const __grid_
         tws[i] = s.tw[i];
         if constexpr (DF) tws_lo[i] = s.tw_lo[i];
     }
+    if (tid == 0) {
+        s_abort = 0;
+        for (int b = 0; b < s.nbuf; ++b) mbar_init(smem_u32(&mbar[b]), 1);
+        fence_mbar_init();
+    }
+    pdl_wait();
     if constexpr (OP == OP_DRIFT) {
         const double2* gbz = s.axy + (s.la3d ? (long)N * N : (long)N);
         for (int i = tid; i < N; i += nthr) bz[i] = gbz[i];
         if (blockIdx.x < s.n_tiles && tid < TX) aslot[tid] = *a_of_tile(blockIdx.x, tid);
     }
     if (tid == 0) {
-        s_abort = 0;
-        for (int b = 0; b < s.nbuf; ++b) mbar_init(smem_u32(&mbar[b]), 1);
-        fence_mbar_init();
         for (int k = 0; k < s.nbuf - 1; ++k) {
             const long id = blockIdx.x + (long)k * gridDim.x;
             if (id < s.n_tiles) issue_load(id, k);
@@ -749,6 +757,7 @@ __global__ void __launch_bounds__(kWpThreads * WPP, 1) k_pencil_wp(const __grid_
         }
         return;
     }
+    pdl_launch();
     if (tid == 0) bulk_wait_all();
     if constexpr (OP == OP_KIN) {
         const double tot = block_reduce<0>(kin, red);
@@ -780,6 +789,7 @@ __global__ void k_poisson_col0(cx_t<R>* vh, const cx_t<R>* tw, const cx_t<R>* tw
     ColAcc<C> macc{sm + gm, 2};
     const long pstride = (long)N * X;
     const long base = (long)y * X;
+    pdl_wait();
     for (int p = t; p < N; p += blockDim.y) acc(p) = vh[base + (long)p * pstride];
     __syncthreads();
     SArgs<R> sa;
