@@ -20,9 +20,10 @@
 // tensor cores with mma.sync m16n8k16 (BF16 in, FP32 accumulate): a block owns
 // an 8 x 8 x 4 brick of sites, stages the brick's periodic halo and the layer's
 // weights in shared memory, and each warp accumulates 32 sites x all output
-// channels over K = 27 offsets x input channels.  Weight gradients are summed
-// over sites with CUDA-core FMAs, 4 x 4 register blocks per thread, per-block
-// partial sums folded in a fixed order (deterministic).
+// channels over K = 27 offsets x input channels; those with 32 outputs run on
+// tcgen05 instead (k_conv_tc).  Weight gradients are tcgen05 GEMMs over the sites
+// (k_wgrad_tc), or CUDA-core FMAs (k_wgrad); per-block partial sums are folded in a
+// fixed order (deterministic).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -246,12 +247,13 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
            ((uint64_t)((sbo >> 4) & 0x3FFF) << 32) | (1ull << 46);
 }
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+template <uint32_t DESC = IDESC>
 __device__ __forceinline__ void mma(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-        ::"r"(tmem_d), "l"(a), "l"(b), "r"(IDESC), "r"(accumulate), "r"(0u)
+        ::"r"(tmem_d), "l"(a), "l"(b), "r"(DESC), "r"(accumulate), "r"(0u)
         : "memory");
 }
 __device__ __forceinline__ void commit(uint32_t bar) {
@@ -298,11 +300,16 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
 
 // X: [S][CIN] bf16; W: [27][32][CIN + 8] bf16 (the packed layer weights);
 // outputs as k_conv.  blockDim 256; grid <= number of bricks.
-template <int CIN>
+// BACK (data gradient of a layer with 32 inputs): the result dA is multiplied by
+// gelu'(Z) of the layer below in the epilogue, rounded to BF16 into ab, and its FP32
+// bias sums go to bpart [gridDim.x][32]; dA itself and an FP32 dZ are never stored
+// (at 128^3 the separate pass took 292 us and 0.94 GB).
+template <int CIN, bool BACK>
 __global__ void __launch_bounds__(256, 2) k_conv_tc(const __nv_bfloat16* __restrict__ X,
                                                     const __nv_bfloat16* __restrict__ W,
                                                     const float* __restrict__ bias, int N, int cout, float* zf,
-                                                    __nv_bfloat16* ab, float* out2, int gelu_ab, int* err) {
+                                                    __nv_bfloat16* ab, float* out2, int gelu_ab,
+                                                    const float* __restrict__ Zb, float* bpart, int* err) {
     // the brick of this kernel (the names shadow the mma.sync kernels' brick)
     constexpr int BX = tc::BX, BY = tc::BY, BZ = tc::BZ, HX = tc::HX, HY = tc::HY, HZ = tc::HZ;
     using G = tc::Geo<CIN>;
@@ -352,6 +359,9 @@ __global__ void __launch_bounds__(256, 2) k_conv_tc(const __nv_bfloat16* __restr
     const int nbx = N / BX, nby = N / BY;
     const long nbricks = (long)nbx * nby * (N / BZ);
     uint32_t phase = 0;
+    float bsum[BACK ? COUT : 1];
+#pragma unroll
+    for (int co = 0; co < (BACK ? COUT : 1); ++co) bsum[co] = 0.f;
     for (long br = blockIdx.x; br < nbricks; br += gridDim.x) {
         const int bxi = (int)(br % nbx), byi = (int)((br / nbx) % nby), bzi = (int)(br / ((long)nbx * nby));
         const int x0 = bxi * BX, y0 = byi * BY, z0 = bzi * BZ;
@@ -396,44 +406,66 @@ __global__ void __launch_bounds__(256, 2) k_conv_tc(const __nv_bfloat16* __restr
             const int r = 32 * q + lane;
             const int x = r % BX, y = r / BX;
             const long gs = ((long)(z0 + zt) * N + (y0 + y)) * N + (x0 + x);
-#pragma unroll
-            for (int co = 0; co < COUT; ++co) v[co] += bs[co];
-            if (cout == COUT) {  // 16-byte stores of the site's 32 channels
-                if (zf) {
-#pragma unroll
-                    for (int j = 0; j < COUT / 4; ++j)
-                        reinterpret_cast<float4*>(zf + gs * COUT)[j] =
-                            make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-                }
-                if (out2) {
-#pragma unroll
-                    for (int j = 0; j < COUT / 4; ++j)
-                        reinterpret_cast<float4*>(out2 + gs * COUT)[j] =
-                            make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-                }
-            } else {
-#pragma unroll
-                for (int co = 0; co < COUT; ++co)
-                    if (co < cout) {
-                        if (zf) zf[gs * cout + co] = v[co];
-                        if (out2) out2[gs * cout + co] = v[co];
-                    }
-            }
-            if (ab) {
+            if constexpr (BACK) {
 #pragma unroll
                 for (int j = 0; j < COUT / 8; ++j) {
+                    const float4 z0v = reinterpret_cast<const float4*>(Zb + gs * COUT)[2 * j];
+                    const float4 z1v = reinterpret_cast<const float4*>(Zb + gs * COUT)[2 * j + 1];
+                    const float zz[8] = {z0v.x, z0v.y, z0v.z, z0v.w, z1v.x, z1v.y, z1v.z, z1v.w};
                     union {
                         __nv_bfloat162 h[4];
                         uint4 u;
                     } pk;
 #pragma unroll
                     for (int q2 = 0; q2 < 4; ++q2) {
-                        const int co = 8 * j + 2 * q2;
-                        const float a0 = co < cout ? (gelu_ab ? gelu(v[co]) : v[co]) : 0.f;
-                        const float a1 = co + 1 < cout ? (gelu_ab ? gelu(v[co + 1]) : v[co + 1]) : 0.f;
-                        pk.h[q2] = __floats2bfloat162_rn(a0, a1);
+                        const float d0 = v[8 * j + 2 * q2] * gelu_grad(zz[2 * q2]);
+                        const float d1 = v[8 * j + 2 * q2 + 1] * gelu_grad(zz[2 * q2 + 1]);
+                        bsum[8 * j + 2 * q2] += d0;
+                        bsum[8 * j + 2 * q2 + 1] += d1;
+                        pk.h[q2] = __floats2bfloat162_rn(d0, d1);
                     }
                     reinterpret_cast<uint4*>(ab + gs * COUT)[j] = pk.u;
+                }
+            } else {
+#pragma unroll
+                for (int co = 0; co < COUT; ++co) v[co] += bs[co];
+                if (cout == COUT) {  // 16-byte stores of the site's 32 channels
+                    if (zf) {
+#pragma unroll
+                        for (int j = 0; j < COUT / 4; ++j)
+                            reinterpret_cast<float4*>(zf + gs * COUT)[j] =
+                                make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+                    }
+                    if (out2) {
+#pragma unroll
+                        for (int j = 0; j < COUT / 4; ++j)
+                            reinterpret_cast<float4*>(out2 + gs * COUT)[j] =
+                                make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+                    }
+                } else {
+#pragma unroll
+                    for (int co = 0; co < COUT; ++co)
+                        if (co < cout) {
+                            if (zf) zf[gs * cout + co] = v[co];
+                            if (out2) out2[gs * cout + co] = v[co];
+                        }
+                }
+                if (ab) {
+#pragma unroll
+                    for (int j = 0; j < COUT / 8; ++j) {
+                        union {
+                            __nv_bfloat162 h[4];
+                            uint4 u;
+                        } pk;
+#pragma unroll
+                        for (int q2 = 0; q2 < 4; ++q2) {
+                            const int co = 8 * j + 2 * q2;
+                            const float a0 = co < cout ? (gelu_ab ? gelu(v[co]) : v[co]) : 0.f;
+                            const float a1 = co + 1 < cout ? (gelu_ab ? gelu(v[co + 1]) : v[co + 1]) : 0.f;
+                            pk.h[q2] = __floats2bfloat162_rn(a0, a1);
+                        }
+                        reinterpret_cast<uint4*>(ab + gs * COUT)[j] = pk.u;
+                    }
                 }
             }
         }
@@ -446,6 +478,23 @@ __global__ void __launch_bounds__(256, 2) k_conv_tc(const __nv_bfloat16* __restr
         mbar_wait(smem_addr(&mbar), phase ^ 1u, 1LL << 32);  // let the timed-out MMAs drain before freeing
     }
     __syncthreads();
+    if constexpr (BACK) {
+        // bias sums: lanes of a warp, then the warps (the weights' shared memory is free now)
+        float* red = reinterpret_cast<float*>(wsm);
+#pragma unroll
+        for (int co = 0; co < COUT; ++co) {
+            float s = bsum[co];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if (lane == 0) red[warp * COUT + co] = s;
+        }
+        __syncthreads();
+        if (tid < COUT) {
+            float s = 0.f;
+            for (int w = 0; w < 8; ++w) s += red[w * COUT + tid];
+            bpart[(long)blockIdx.x * COUT + tid] = s;
+        }
+    }
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)TMEM_COLS)
                      : "memory");
@@ -534,61 +583,69 @@ __global__ void __launch_bounds__(256) k_wgrad(const __nv_bfloat16* __restrict__
 }
 
 // Weight gradient on the tensor cores (tcgen05), the same sums as k_wgrad:
-//   dW[o][ci][co] = sum_s A[s + o][ci] dZ[s][co],  db[co] = sum_s dZ[s][co].
-// Per 8 x 8 x 4 brick (K = 256 sites) and per group of OPG = 128 / CINP
-// offsets, the block builds the group's shifted activations as the A operand
-// [128 rows (offset j, channel ci)] x [256 sites] in the canonical no-swizzle
-// K-major layout (core matrix (row group, 8-site chunk) at (rg * 32 + chunk) *
-// 128 B), and dZ of the brick once as the B operand [32 outputs] x [256 sites]
-// (BF16, the same layout); one thread issues 16 MMAs of M = 128, N = 32, K = 16
-// into the group's 32 tensor-memory columns, accumulating over every brick the
-// block processes.  Two group buffers alternate, so the next group is built
-// while the previous group's MMAs run; an mbarrier per buffer orders reuse.
-// dZ is rounded to BF16 for the tensor cores (the activations already are);
-// the bias gradient stays an FP32 sum.  Waits are bounded; tensor memory is
-// freed on every path.  partial: as k_wgrad.
+//   dW[o][ci][co] = sum_s A[s + o][ci] dZ[s][co].
+// Sites are the K dimension of the GEMM, and activations and dZ (BF16) are
+// channel-last, so both operands are MN-major as they lie in memory.  In the
+// canonical no-swizzle MN-major layout a core matrix is 8 sites x 8 channels, 16
+// bytes per site, 128 contiguous bytes: exactly the 8 sites x = 0..7 of one (y, z)
+// row and one channel chunk of a halo stored [hz][hy][chunk][hx][8 channels], for
+// any x shift.  Nothing is transposed or copied per offset:
+//   A  K step (next 8 sites) = next y row, LBO = KC HX 16 B; M step (next 8
+//      channels) = next chunk, SBO = HX 16 B.  Since a row holds KC chunks, the M
+//      groups run on into the rows y + 1, y + 2, ...: the 128 M rows are the
+//      channels at the shifts dy = -1, 0, 1 and the rows beyond (ignored; their
+//      reads stay inside the block's shared memory).  The (dz, dx) shift is the
+//      start address.
+//   B  dZ stored [row][chunk][x][8 channels]: LBO = NC / 8 * 128 B, SBO = 128 B.
+// Per 8 x 8 x 4 brick (K = 256 sites) one thread issues 16 MMAs (M = 128, N = NC, K
+// = 16) into each of 9 accumulators of NC tensor-memory columns, which add up over
+// all bricks of the block.  Bricks arrive by cp.async in a ring of three: while
+// the MMAs of brick k run, brick k + 1 is there and k + 2 is under way.  Bound by the
+// MMAs' reads of A (82 cycles for 4 KB).  Building each offset group's shifted
+// operand through registers instead was bound by that copy: at 128^3, us, 32 -> 32
+// layer 1442 -> 344, 4 -> 32 876 -> 303, 32 -> 2 1488 -> 318.  Waits are bounded;
+// tensor memory is freed on every path.  partial: [gridDim.x][27 * cin * cout].
 namespace wtc {
-constexpr int K = BSITES;            // 256 sites per brick
-constexpr int KCH = K / 8;           // 32 chunks of 8 sites
-constexpr int OPER_BYTES = 128 * K * 2;  // one A operand: 64 KB
-constexpr int DZ_BYTES = 32 * K * 2;     // B operand: 16 KB
-constexpr uint32_t LBO = 128, SBO = KCH * 128;
-template <int CINP> struct Geo {
-    static constexpr int OPG = 128 / CINP;                    // offsets per group
-    static constexpr int NGROUPS = (KOFF + OPG - 1) / OPG;    // 7 (CINP 32) or 4 (CINP 16)
-    static constexpr int HALO_BYTES = HALO * CINP * 2;
-    static constexpr size_t SMEM = 2 * (size_t)OPER_BYTES + DZ_BYTES + HALO_BYTES + 128;
-    static constexpr uint32_t TMEM_COLS = NGROUPS * 32 <= 128 ? 128 : 256;
+constexpr int STAGES = 3;
+constexpr int ROWS = BY * BZ;  // rows of 8 sites in a brick
+template <int CINP, int NC> struct Geo {
+    static constexpr int KC = CINP / 8;                      // 16-byte channel chunks per site
+    static constexpr int HALO_BYTES = HZ * HY * KC * HX * 16;  // 38,400 for CINP = 32
+    static constexpr int DZ_BYTES = ROWS * (NC / 8) * 128;     // 16,384 for NC = 32
+    static constexpr int STAGE_BYTES = HALO_BYTES + DZ_BYTES;
+    // the M rows beyond dy = 1 of the last row read at most 16 chunks past it
+    static constexpr size_t SMEM = (size_t)STAGES * STAGE_BYTES + 16 * HX * 16 + 128;
+    static constexpr uint32_t LBO_A = KC * HX * 16, SBO_A = HX * 16;
+    static constexpr uint32_t LBO_B = NC / 8 * 128, SBO_B = 128;
+    static constexpr uint32_t TMEM_COLS = 9 * NC <= 256 ? 256 : 512;
+    // D FP32, A and B BF16, both MN-major (bits 15, 16), N >> 3, M >> 4
+    static constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) |
+                                      ((uint32_t)(NC >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+    static_assert(HALO_BYTES % 128 == 0 && DZ_BYTES % 128 == 0, "operand alignment");
 };
 }  // namespace wtc
 
-template <int CINP>
-__global__ void __launch_bounds__(256, 1) k_wgrad_tc(const __nv_bfloat16* __restrict__ A, const float* __restrict__ dZ,
-                                                     int N, int cin, int cout, float* partial, int* err) {
-    using G = wtc::Geo<CINP>;
-    constexpr int OPG = G::OPG, NG = G::NGROUPS;
+template <int CINP, int NC>
+__global__ void __launch_bounds__(256, 1) k_wgrad_tc(const __nv_bfloat16* __restrict__ A,
+                                                     const __nv_bfloat16* __restrict__ dZ, int N, int cin, int cout,
+                                                     float* partial, int* err) {
+    using G = wtc::Geo<CINP, NC>;
+    constexpr int KC = G::KC;
     using tc::commit;
     using tc::fence_after;
     using tc::fence_before;
     using tc::mbar_init;
     using tc::mbar_wait;
-    using tc::mma;
     using tc::proxy_fence;
     using tc::smem_addr;
     using tc::smem_desc;
     extern __shared__ __align__(128) unsigned char smem_w[];
-    __shared__ __align__(8) uint64_t mbar[2];
+    __shared__ __align__(8) uint64_t mbar[wtc::STAGES];
     __shared__ uint32_t tmem_slot;
-    __shared__ float bred[8][32];
     unsigned char* base = smem_align128(smem_w);
-    unsigned char* oper[2] = {base, base + wtc::OPER_BYTES};
-    unsigned char* dzb = base + 2 * wtc::OPER_BYTES;
-    __nv_bfloat16* halo = reinterpret_cast<__nv_bfloat16*>(dzb + wtc::DZ_BYTES);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    if (tid == 0) {
-        mbar_init(smem_addr(&mbar[0]));
-        mbar_init(smem_addr(&mbar[1]));
-    }
+    if (tid == 0)
+        for (int i = 0; i < wtc::STAGES; ++i) mbar_init(smem_addr(&mbar[i]));
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_slot)),
                      "r"(G::TMEM_COLS)
@@ -602,144 +659,128 @@ __global__ void __launch_bounds__(256, 1) k_wgrad_tc(const __nv_bfloat16* __rest
 
     const int nbx = N / BX, nby = N / BY, nbz = N / BZ;
     const int nbricks = nbx * nby * nbz;
-    int ncommit[2] = {0, 0};  // commits issued on each buffer (the same in every thread)
-    int last = -1;            // buffer of the latest commit
-    float bsum = 0.f;         // bias partial of output tid % 32
-    bool first = true;
-    int fail = 0;             // this thread's wait timed out; combined at block barriers
-    auto wait_buf = [&](int b, long long limit) {
-        if (ncommit[b] > 0 && !mbar_wait(smem_addr(&mbar[b]), (uint32_t)((ncommit[b] - 1) & 1), limit)) fail = 1;
-    };
-    bool abort = false;
-    for (int br = blockIdx.x; br < nbricks && !abort; br += gridDim.x) {
-        const int bxi = br % nbx, byi = (br / nbx) % nby, bzi = br / (nbx * nby);
-        const int x0 = bxi * BX, y0 = byi * BY, z0 = bzi * BZ;
-        // the previous brick's MMAs read the halo, dZ and both buffers: wait for the last commit
-        if (last >= 0) wait_buf(last, 1LL << 31);
-        fence_after();
-        // periodic halo [hz][hy][hx][CINP] (16-byte copies)
-        for (int i = tid; i < HALO * (CINP / 8); i += blockDim.x) {
-            const int h = i / (CINP / 8), c = i % (CINP / 8);
-            const int hx = h % HX, hy = (h / HX) % HY, hz = h / (HX * HY);
-            const long gs = ((long)wrapi(z0 + hz - 1, N) * N + wrapi(y0 + hy - 1, N)) * N + wrapi(x0 + hx - 1, N);
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(halo + (size_t)h * CINP + c * 8)),
-                         "l"(A + gs * CINP + c * 8)
-                         : "memory");
-        }
-        // dZ of the brick -> B operand: output co, chunk r = y + 8 z of 8 sites x = 0..7
-        for (int q = tid; q < 32 * wtc::KCH; q += blockDim.x) {
-            const int co = q % 32, r = q / 32;
-            const int y = r % BY, z = r / BY;
-            union {
-                __nv_bfloat162 h[4];
-                uint4 u;
-            } pk;
-#pragma unroll
-            for (int x2 = 0; x2 < 4; ++x2) {
-                float v0 = 0.f, v1 = 0.f;
-                if (co < cout) {
-                    const long g0 = ((long)(z0 + z) * N + (y0 + y)) * N + (x0 + 2 * x2);
-                    v0 = dZ[g0 * cout + co];
-                    v1 = dZ[(g0 + 1) * cout + co];
-                    bsum += v0 + v1;
-                }
-                pk.h[x2] = __floats2bfloat162_rn(v0, v1);
+    const int mine = blockIdx.x < nbricks ? (nbricks - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
+    // copy the k-th brick of this block into its stage (one cp.async group, empty past the end)
+    auto load = [&](int k) {
+        if (k < mine) {
+            const int br = blockIdx.x + k * gridDim.x;
+            const int bxi = br % nbx, byi = (br / nbx) % nby, bzi = br / (nbx * nby);
+            const int x0 = bxi * BX, y0 = byi * BY, z0 = bzi * BZ;
+            const uint32_t st = smem_addr(base) + (uint32_t)((k % wtc::STAGES) * G::STAGE_BYTES);
+            for (int i = tid; i < HZ * HY * KC * HX; i += blockDim.x) {
+                const int hx = i % HX, ch = (i / HX) % KC, hy = (i / (HX * KC)) % HY, hz = i / (HX * KC * HY);
+                const long gs = ((long)wrapi(z0 + hz - 1, N) * N + wrapi(y0 + hy - 1, N)) * N + wrapi(x0 + hx - 1, N);
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(st + (uint32_t)i * 16),
+                             "l"(A + gs * CINP + ch * 8)
+                             : "memory");
             }
-            *reinterpret_cast<uint4*>(dzb + (size_t)((co / 8) * wtc::KCH + r) * 128 + (co % 8) * 16) = pk.u;
+            for (int i = tid; i < wtc::ROWS * (NC / 8) * 8; i += blockDim.x) {  // [row][x][chunk] reads whole lines
+                const int ch = i % (NC / 8), x = (i / (NC / 8)) % 8, r = i / NC;
+                const long gs = ((long)(z0 + r / BY) * N + (y0 + r % BY)) * N + (x0 + x);
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(st + (uint32_t)(G::HALO_BYTES +
+                                                                                (r * (NC / 8) + ch) * 128 + x * 16)),
+                             "l"(dZ + gs * NC + ch * 8)
+                             : "memory");
+            }
         }
-        asm volatile("cp.async.wait_all;" ::: "memory");
-        if (__syncthreads_or(fail)) {
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    int fail = 0;  // this thread's wait timed out; combined at block barriers
+    bool abort = false;
+    auto wait_brick = [&](int k, long long limit) {  // the MMAs of brick k are done
+        if (k >= 0 && !mbar_wait(smem_addr(&mbar[k % wtc::STAGES]), (uint32_t)((k / wtc::STAGES) & 1), limit)) fail = 1;
+    };
+    load(0);
+    load(1);
+    int issued = 0;  // bricks whose MMAs have been issued
+    for (int k = 0; k < mine; ++k) {
+        asm volatile("cp.async.wait_group 1;" ::: "memory");  // brick k has arrived (this thread's part)
+        proxy_fence();
+        if (__syncthreads_or(fail)) {  // the same decision in every thread
             abort = true;
             break;
         }
-        for (int g = 0; g < NG; ++g) {
-            const int b = (ncommit[0] + ncommit[1]) & 1;
-            wait_buf(b, 1LL << 31);  // this buffer's previous MMAs are done
+        if (tid == 0) {
             fence_after();
-            unsigned char* op = oper[b];
-            // rows m = j CINP + ci (offset o = g OPG + j), chunk r: the 8 sites
-            // x = 0..7 of row (y, z) shifted by the offset
-            for (int q = tid; q < 128 * wtc::KCH; q += blockDim.x) {
-                const int ci = q % CINP, rest = q / CINP;
-                const int r = rest % wtc::KCH, j = rest / wtc::KCH;
-                const int o = g * OPG + j;
-                const int y = r % BY, z = r / BY;
-                union {
-                    __nv_bfloat16 h[8];
-                    uint4 u;
-                } pk;
-                if (o < KOFF) {
-                    const int hb = (1 + off_dx(o)) + HX * ((1 + y + off_dy(o)) + HY * (1 + z + off_dz(o)));
-#pragma unroll
-                    for (int x = 0; x < 8; ++x) pk.h[x] = halo[(size_t)(hb + x) * CINP + ci];
-                } else {
-                    pk.u = make_uint4(0u, 0u, 0u, 0u);
-                }
-                const int m = j * CINP + ci;
-                *reinterpret_cast<uint4*>(op + (size_t)((m / 8) * wtc::KCH + r) * 128 + (m % 8) * 16) = pk.u;
-            }
-            proxy_fence();  // generic-proxy shared writes -> visible to the tensor cores
-            if (__syncthreads_or(fail)) {  // the same decision in every thread
-                abort = true;
-                break;
-            }
-            if (tid == 0) {
-                fence_after();
-                const uint32_t a0 = smem_addr(op), b0 = smem_addr(dzb);
+            const uint32_t h0 = smem_addr(base) + (uint32_t)((k % wtc::STAGES) * G::STAGE_BYTES), d0 = h0 + G::HALO_BYTES;
 #pragma unroll 1
-                for (int kk = 0; kk < wtc::KCH / 2; ++kk)
-                    mma(tmem + (uint32_t)(g * 32), smem_desc(a0 + (uint32_t)(2 * kk * 128), wtc::LBO, wtc::SBO),
-                        smem_desc(b0 + (uint32_t)(2 * kk * 128), wtc::LBO, wtc::SBO), (!first || kk > 0) ? 1u : 0u);
-                commit(smem_addr(&mbar[b]));
+            for (int r = 0; r < wtc::ROWS; r += 2) {  // rows y, y + 1 of plane z
+                const int y = r % BY, z = r / BY;
+                const uint64_t bd = smem_desc(d0 + (uint32_t)(r * (NC / 8) * 128), G::LBO_B, G::SBO_B);
+#pragma unroll
+                for (int q = 0; q < 9; ++q) {  // (dz, dx) = (q / 3 - 1, q % 3 - 1); start row dy = -1
+                    const uint32_t ad = h0 + (uint32_t)((((z + q / 3) * HY + y) * KC * HX + q % 3) * 16);
+                    tc::mma<G::IDESC>(tmem + (uint32_t)(q * NC), smem_desc(ad, G::LBO_A, G::SBO_A), bd,
+                                      (k > 0 || r > 0) ? 1u : 0u);
+                }
             }
-            ++ncommit[b];
-            last = b;
+            commit(smem_addr(&mbar[k % wtc::STAGES]));
         }
-        first = false;
+        issued = k + 1;
+        // the stage of brick k + 2 is that of brick k - 1, whose MMAs run before these
+        wait_brick(k - 1, 1LL << 31);
+        load(k + 2);
     }
-    // every MMA done before the accumulators are read (after a time-out: a
-    // longer bounded wait, so the MMAs in flight drain before tensor memory
-    // is freed)
-    if (last >= 0) wait_buf(last, abort ? (1LL << 32) : (1LL << 31));
-    if (last >= 0) wait_buf(last ^ 1, abort ? (1LL << 32) : (1LL << 31));
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    // every MMA done before the accumulators are read (after a time-out: a longer
+    // bounded wait, so that those in flight drain before tensor memory is freed)
+    wait_brick(issued - 1, abort ? (1LL << 32) : (1LL << 31));
     fence_after();
     if (__syncthreads_or(fail)) abort = true;
     const int nw = KOFF * cin * cout;
-    float* outp = partial + (long)blockIdx.x * (nw + cout);
+    float* outp = partial + (long)blockIdx.x * nw;
+    // accumulator row m = channel m % CINP at dy = m / CINP - 1; warps w and w + 4 read
+    // rows 32 (w % 4) .. of accumulators 0, 2, .. and 1, 3, ..
     if (!abort) {
-        // warp w reads lanes 32 (w % 4) .. of groups w / 4, w / 4 + 2, ...
-        for (int g = warp >> 2; g < NG; g += 2) {
+        const int m = 32 * (warp & 3) + lane;
+        const int ci = m % CINP, dyi = m / CINP;
+        for (int q = warp >> 2; q < 9; q += 2) {
             float v[32];
-            tc::tmem_ld32(tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(g * 32), v);
-            const int m = 32 * (warp & 3) + lane;
-            const int o = g * OPG + m / CINP, ci = m % CINP;
-            if (o < KOFF && ci < cin && !first) {
-                for (int co = 0; co < cout; ++co) outp[(o * cin + ci) * cout + co] = v[co];
-            } else if (o < KOFF && ci < cin) {  // no brick: zero partial
-                for (int co = 0; co < cout; ++co) outp[(o * cin + ci) * cout + co] = 0.f;
-            }
+            tc::tmem_ld32(tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(q * NC), v);
+            const int o = (q / 3) * 9 + dyi * 3 + q % 3;
+            if (dyi < 3 && ci < cin)
+#pragma unroll
+                for (int co = 0; co < NC; ++co)
+                    if (co < cout) outp[(o * cin + ci) * cout + co] = mine > 0 ? v[co] : 0.f;
         }
     }
-    bred[warp][lane] = bsum;
     fence_before();
     __syncthreads();
-    if (tid < cout) {
-        float s = 0.f;
-        for (int w = 0; w < 8; ++w) s += bred[w][tid];
-        outp[nw + tid] = s;
-    }
     if (abort && tid == 0) atomicExch(err, 1);
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(G::TMEM_COLS) : "memory");
 }
 
-// fixed-order fold of per-block partials: out[i] = sum_b partial[b][i] (FP64 sum)
-__global__ void k_fold(const float* partial, int nblk, int n, float* out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+// bias gradient partials: part[block][c] = sum of this block's sites of dZ [S][c] (FP32)
+__global__ void __launch_bounds__(256) k_bias(const float* dZ, long S, int c, float* part) {
+    __shared__ float red[256];
+    const int per = 256 / c, ch = threadIdx.x % c, slot = threadIdx.x / c;  // c divides 256 (2, 4, 32)
+    float s = 0.f;
+    for (long i = (long)blockIdx.x * per + slot; i < S; i += (long)gridDim.x * per) s += dZ[i * c + ch];
+    red[threadIdx.x] = s;
+    __syncthreads();
+    for (int w = per / 2; w > 0; w >>= 1) {
+        if (slot < w) red[threadIdx.x] += red[threadIdx.x + w * c];
+        __syncthreads();
+    }
+    if (slot == 0) part[(long)blockIdx.x * c + ch] = red[threadIdx.x];
+}
+
+// fixed-order fold of per-block partials: out[i] = sum_b partial[b][i] (FP64 sum);
+// 32 outputs x 8 slices of the blocks per block of 256 threads
+__global__ void __launch_bounds__(256) k_fold(const float* partial, int nblk, int n, float* out) {
+    __shared__ double red[8][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int i = blockIdx.x * 32 + lane;
     double s = 0.0;
-    for (int b = 0; b < nblk; ++b) s += partial[(long)b * n + i];
-    out[i] = (float)s;
+    if (i < n)
+        for (int b = w; b < nblk; b += 8) s += partial[(long)b * n + i];
+    red[w][lane] = s;
+    __syncthreads();
+    if (w == 0 && i < n) {
+        for (int k = 1; k < 8; ++k) s += red[k][lane];
+        out[i] = (float)s;
+    }
 }
 
 // input features [S][16] bf16: Re psi, Im psi, V / v_scale, |psi|^2 - 1, zeros
@@ -800,13 +841,19 @@ __global__ void k_gelu_back(const float* dA, const float* Z, long S, int c, int 
     dZb[i] = __float2bfloat16(v);
 }
 
-// dY [S][2] FP32 -> bf16 [S][16] (the data-gradient conv input)
-__global__ void k_pad16(const float* dY, long S, int c, __nv_bfloat16* out) {
-    const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (i >= S * 16) return;
-    const long s = i / 16;
-    const int ch = (int)(i % 16);
-    out[i] = __float2bfloat16(ch < c ? dY[s * c + ch] : 0.f);
+// dY [S][2] FP32 -> bf16 [S][16] (the data-gradient conv input), one site per thread
+__global__ void k_pad16(const float2* dY, long S, uint4* out) {
+    const long s = blockIdx.x * (long)blockDim.x + threadIdx.x;
+    if (s >= S) return;
+    const float2 d = dY[s];
+    union {
+        __nv_bfloat162 h[4];
+        uint4 u;
+    } w;
+    w.u = make_uint4(0u, 0u, 0u, 0u);
+    w.h[0] = __floats2bfloat162_rn(d.x, d.y);
+    out[2 * s] = w.u;
+    out[2 * s + 1] = make_uint4(0u, 0u, 0u, 0u);
 }
 
 // psi += tau * Y
@@ -924,16 +971,20 @@ class Corrector {
                                      (int)ConvSmem<32, 32>::bytes()));
         NN_CUDA(cudaFuncSetAttribute(k_conv<32, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)ConvSmem<32, 8>::bytes()));
-        NN_CUDA(cudaFuncSetAttribute(k_conv_tc<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::Geo<32>::SMEM));
-        NN_CUDA(cudaFuncSetAttribute(k_conv_tc<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::Geo<16>::SMEM));
+        for (auto* k : {k_conv_tc<32, false>, k_conv_tc<32, true>})
+            NN_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::Geo<32>::SMEM));
+        for (auto* k : {k_conv_tc<16, false>, k_conv_tc<16, true>})
+            NN_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::Geo<16>::SMEM));
         errb_.alloc(sizeof(int));
         NN_CUDA(cudaMemset(errb_.p, 0, sizeof(int)));
         NN_CUDA(cudaFuncSetAttribute(k_wgrad<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wgrad_smem(16, 32)));
         NN_CUDA(cudaFuncSetAttribute(k_wgrad<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wgrad_smem(32, 32)));
-        NN_CUDA(cudaFuncSetAttribute(k_wgrad_tc<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)wtc::Geo<32>::SMEM));
-        NN_CUDA(cudaFuncSetAttribute(k_wgrad_tc<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)wtc::Geo<16>::SMEM));
+        NN_CUDA(cudaFuncSetAttribute(k_wgrad_tc<32, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)wtc::Geo<32, 16>::SMEM));
+        NN_CUDA(cudaFuncSetAttribute(k_wgrad_tc<32, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)wtc::Geo<32, 32>::SMEM));
+        NN_CUDA(cudaFuncSetAttribute(k_wgrad_tc<16, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)wtc::Geo<16, 32>::SMEM));
     }
     ~Corrector() {
         if (st_) {
@@ -1013,20 +1064,17 @@ class Corrector {
         k_mse<<<nb, 256, 0, st_>>>(Y_.as<float>(), T_.as<float>(), 2 * S, (float)(1.0 / (2.0 * S)), dY_.as<float>(),
                                    lossp_.as<double>());
         // layer 3: dZ3 = dY (linear)
-        wgrad<32>(A2_.as<__nv_bfloat16>(), dY_.as<float>(), layers_[2]);
         dYb_.alloc(sizeof(__nv_bfloat16) * 16 * S);
-        k_pad16<<<(unsigned)((S * 16 + 255) / 256), 256, 0, st_>>>(dY_.as<float>(), S, 2, dYb_.as<__nv_bfloat16>());
-        dA_.alloc(sizeof(float) * 32 * S);
-        conv_bwd<16, 32>(dYb_.as<__nv_bfloat16>(), layers_[2], dA_.as<float>());  // dA2 = conv^T(dZ3)
-        dZ_.alloc(sizeof(float) * 32 * S);
+        k_pad16<<<(unsigned)((S + 255) / 256), 256, 0, st_>>>(dY_.as<float2>(), S, dYb_.as<uint4>());
+        wgrad<32, 16>(A2_.as<__nv_bfloat16>(), dY_.as<float>(), dYb_.as<__nv_bfloat16>(), layers_[2]);
         dZb_.alloc(sizeof(__nv_bfloat16) * 32 * S);
-        k_gelu_back<<<(unsigned)((S * 32 + 255) / 256), 256, 0, st_>>>(dA_.as<float>(), Z2_.as<float>(), S, 32, 32,
-                                                                         dZ_.as<float>(), dZb_.as<__nv_bfloat16>());
-        wgrad<32>(A1_.as<__nv_bfloat16>(), dZ_.as<float>(), layers_[1]);
-        conv_bwd<32, 32>(dZb_.as<__nv_bfloat16>(), layers_[1], dA_.as<float>());  // dA1 = conv^T(dZ2)
-        k_gelu_back<<<(unsigned)((S * 32 + 255) / 256), 256, 0, st_>>>(dA_.as<float>(), Z1_.as<float>(), S, 32, 32,
-                                                                         dZ_.as<float>(), dZb_.as<__nv_bfloat16>());
-        wgrad<16>(X0_.as<__nv_bfloat16>(), dZ_.as<float>(), layers_[0]);
+        // dA2 = conv^T(dZ3), dZ2 = dA2 gelu'(Z2)
+        back<16>(dYb_.as<__nv_bfloat16>(), layers_[2], Z2_.as<float>(), dZb_, layers_[1]);
+        wgrad<32, 32>(A1_.as<__nv_bfloat16>(), dZ_.as<float>(), dZb_.as<__nv_bfloat16>(), layers_[1]);
+        dZb2_.alloc(sizeof(__nv_bfloat16) * 32 * S);
+        // dA1 = conv^T(dZ2), dZ1 = dA1 gelu'(Z1)
+        back<32>(dZb_.as<__nv_bfloat16>(), layers_[1], Z1_.as<float>(), dZb2_, layers_[0]);
+        wgrad<16, 32>(X0_.as<__nv_bfloat16>(), dZ_.as<float>(), dZb2_.as<__nv_bfloat16>(), layers_[0]);
         NN_CUDA(cudaGetLastError());
         std::vector<double> lp(nb);
         NN_CUDA(cudaMemcpyAsync(lp.data(), lossp_.p, sizeof(double) * nb, cudaMemcpyDeviceToHost, st_));
@@ -1101,18 +1149,22 @@ class Corrector {
     }
     // CIN -> 32 layers on the tcgen05 kernel (grids N % 16 == 0), the others on mma.sync
     bool tc_ok() const { return use_tc_ && N_ % tc::BY == 0; }
+    // two blocks per SM (the kernel's launch bounds; the shared-memory carve-out is
+    // set at launch), so one block's MMAs overlap the other's halo loads and epilogue
+    unsigned conv_blocks() const {
+        return (unsigned)std::min<long>(S_ / (tc::BX * tc::BY * tc::BZ), 2L * sms());
+    }
+    static int sms() {
+        int dev = 0, n = 148;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        return n;
+    }
     template <int CIN>
     void conv_tc(const __nv_bfloat16* X, const __nv_bfloat16* W, const float* bias, int cout, float* zf,
                  __nv_bfloat16* ab, float* out2, bool gelu_ab) {
-        int dev = 0, sms = 148;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        // two blocks per SM (the kernel's launch bounds; the shared-memory carve-out is
-        // set at launch), so one block's MMAs overlap the other's halo loads and epilogue
-        const long nbricks = S_ / (tc::BX * tc::BY * tc::BZ);
-        const unsigned blocks = (unsigned)std::min<long>(nbricks, 2L * sms);
-        k_conv_tc<CIN><<<blocks, 256, tc::Geo<CIN>::SMEM, st_>>>(X, W, bias, N_, cout, zf, ab, out2, gelu_ab ? 1 : 0,
-                                                                 errb_.as<int>());
+        k_conv_tc<CIN, false><<<conv_blocks(), 256, tc::Geo<CIN>::SMEM, st_>>>(
+            X, W, bias, N_, cout, zf, ab, out2, gelu_ab ? 1 : 0, nullptr, nullptr, errb_.as<int>());
     }
     template <int CINP, int COUTP>
     void conv(const __nv_bfloat16* X, Layer& L, float* zf, __nv_bfloat16* ab, float* out2, bool gelu_ab) {
@@ -1126,37 +1178,58 @@ class Corrector {
         k_conv<CINP, COUTP><<<blocks, 256, ConvSmem<CINP, COUTP>::bytes(), st_>>>(
             X, L.fwd.as<__nv_bfloat16>(), L.db.as<float>(), N_, L.cout, zf, ab, out2, gelu_ab ? 1 : 0);
     }
-    // data gradient: input channels = the layer's outputs (padded to CINP), outputs = its inputs
-    template <int CINP, int COUTP>
-    void conv_bwd(const __nv_bfloat16* dZb, Layer& L, float* dA) {
-        if constexpr ((CINP == 32 || CINP == 16) && COUTP == 32) {
-            if (tc_ok()) {
-                conv_tc<CINP>(dZb, L.bwd.as<__nv_bfloat16>(), nullptr, L.cin, dA, nullptr, nullptr, false);
-                return;
-            }
-        }
-        const unsigned blocks = (unsigned)(S_ / BSITES);
-        k_conv<CINP, COUTP><<<blocks, 256, ConvSmem<CINP, COUTP>::bytes(), st_>>>(
-            dZb, L.bwd.as<__nv_bfloat16>(), nullptr, N_, L.cin, dA, nullptr, nullptr, 0);
-    }
+    // Through layer L and the GELU below it: out = bf16(conv^T(dZb) gelu'(Z)) (input
+    // channels = the layer's outputs, padded to CINP), and the bias gradient of the
+    // layer `below` where the tensor path computes the weight gradients; elsewhere
+    // the FP32 dZ_ is left for wgrad.
     template <int CINP>
-    void wgrad(const __nv_bfloat16* A, const float* dZ, Layer& L) {
-        int dev = 0, sms = 148;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    void back(const __nv_bfloat16* dZb, Layer& L, const float* Z, DBuf& out, Layer& below) {
+        const long S = S_;
+        if (tc_ok()) {
+            const unsigned blocks = conv_blocks();
+            bpart_.alloc(sizeof(float) * 32 * blocks);
+            k_conv_tc<CINP, true><<<blocks, 256, tc::Geo<CINP>::SMEM, st_>>>(
+                dZb, L.bwd.as<__nv_bfloat16>(), nullptr, N_, L.cin, nullptr, out.as<__nv_bfloat16>(), nullptr, 0, Z,
+                bpart_.as<float>(), errb_.as<int>());
+            k_fold<<<1, 256, 0, st_>>>(bpart_.as<float>(), (int)blocks, 32, below.gb.as<float>());
+            return;
+        }
+        dA_.alloc(sizeof(float) * 32 * S);
+        dZ_.alloc(sizeof(float) * 32 * S);
+        const unsigned blocks = (unsigned)(S_ / BSITES);
+        k_conv<CINP, 32><<<blocks, 256, ConvSmem<CINP, 32>::bytes(), st_>>>(
+            dZb, L.bwd.as<__nv_bfloat16>(), nullptr, N_, L.cin, dA_.as<float>(), nullptr, nullptr, 0);
+        k_gelu_back<<<(unsigned)((S * 32 + 255) / 256), 256, 0, st_>>>(dA_.as<float>(), Z, S, 32, 32, dZ_.as<float>(),
+                                                                         out.as<__nv_bfloat16>());
+        if (use_tc_) bias_sum(dZ_.as<float>(), below);
+    }
+    void bias_sum(const float* dZ, Layer& L) {
+        const int blocks = 2 * sms();
+        bpart_.alloc(sizeof(float) * (size_t)blocks * L.cout);
+        k_bias<<<blocks, 256, 0, st_>>>(dZ, S_, L.cout, bpart_.as<float>());
+        k_fold<<<1, 256, 0, st_>>>(bpart_.as<float>(), blocks, L.cout, L.gb.as<float>());
+    }
+    // weight gradient of layer L from its input A and dZ: on the tensor cores from
+    // the BF16 dZb [S][NC] (one block per SM; the bias gradient of all but the last
+    // layer comes with back()), or the CUDA-core sums of the FP32 dZ (set_tensor_path(0))
+    template <int CINP, int NC>
+    void wgrad(const __nv_bfloat16* A, const float* dZ, const __nv_bfloat16* dZb, Layer& L) {
         const int nbricks = (int)(S_ / BSITES);
         const int nw = KOFF * L.cin * L.cout;
-        // tensor cores (one block per SM, shared memory for two operand buffers),
-        // or the CUDA-core sums (set_tensor_path(0))
-        const int nblk = use_tc_ ? std::min(nbricks, sms) : std::min(nbricks, 2 * sms);
+        if (use_tc_) {
+            const int nblk = std::min(nbricks, sms());
+            part_.alloc(sizeof(float) * (size_t)nblk * nw);
+            k_wgrad_tc<CINP, NC><<<nblk, 256, wtc::Geo<CINP, NC>::SMEM, st_>>>(A, dZb, N_, L.cin, L.cout,
+                                                                               part_.as<float>(), errb_.as<int>());
+            k_fold<<<(nw + 31) / 32, 256, 0, st_>>>(part_.as<float>(), nblk, nw, L.gw.as<float>());
+            if (L.cout == 2) bias_sum(dZ, L);
+            return;
+        }
+        const int nblk = std::min(nbricks, 2 * sms());
         part_.alloc(sizeof(float) * (size_t)nblk * (nw + L.cout));
-        if (use_tc_)
-            k_wgrad_tc<CINP><<<nblk, 256, wtc::Geo<CINP>::SMEM, st_>>>(A, dZ, N_, L.cin, L.cout, part_.as<float>(),
-                                                                       errb_.as<int>());
-        else
-            k_wgrad<CINP><<<nblk, 256, wgrad_smem(CINP, L.cout), st_>>>(A, dZ, N_, L.cin, L.cout, part_.as<float>());
+        k_wgrad<CINP><<<nblk, 256, wgrad_smem(CINP, L.cout), st_>>>(A, dZ, N_, L.cin, L.cout, part_.as<float>());
         fold_.alloc(sizeof(float) * (nw + L.cout));
-        k_fold<<<(nw + L.cout + 255) / 256, 256, 0, st_>>>(part_.as<float>(), nblk, nw + L.cout, fold_.as<float>());
+        k_fold<<<(nw + L.cout + 31) / 32, 256, 0, st_>>>(part_.as<float>(), nblk, nw + L.cout, fold_.as<float>());
         NN_CUDA(cudaMemcpyAsync(L.gw.p, fold_.p, sizeof(float) * nw, cudaMemcpyDeviceToDevice, st_));
         NN_CUDA(cudaMemcpyAsync(L.gb.p, fold_.as<float>() + nw, sizeof(float) * L.cout, cudaMemcpyDeviceToDevice, st_));
     }
@@ -1199,7 +1272,7 @@ class Corrector {
     Layer layers_[3];
     double v_scale_ = 1.0, tau_ = 1.0;
     long t_ = 0;
-    DBuf X0_, A1_, A2_, Z1_, Z2_, Y_, T_, dY_, dYb_, dA_, dZ_, dZb_, lossp_, part_, fold_;
+    DBuf X0_, A1_, A2_, Z1_, Z2_, Y_, T_, dY_, dYb_, dA_, dZ_, dZb_, dZb2_, lossp_, part_, fold_, bpart_;
     DBuf errb_;           // device flag: a bounded wait of the tcgen05 kernel timed out
     bool use_tc_ = true;
 };
