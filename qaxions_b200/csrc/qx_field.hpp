@@ -151,7 +151,7 @@ class Field {
     void half_kick() { kick(0.5 * ds_); }
     void full_kick() { kick(ds_); }
     void drift_update();
-    void propagate();
+    virtual void propagate() = 0;
     // merged leapfrog of src/main.cxx:64-85 (measurements off), fused passes,
     // loop body replayed from a CUDA graph
     virtual void step(int nsteps) = 0;

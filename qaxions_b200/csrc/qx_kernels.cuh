@@ -296,8 +296,12 @@ __device__ __forceinline__ cx_t<R>* x_setup(const XArgs<R>& a, unsigned char* sm
     return tN + x_table_elems<N, R>() + threadIdx.y * row_smem_elems(N);
 }
 
-// first row of this thread's row slot and the row stride of the grid
-__device__ __forceinline__ long x_row0() { return (long)blockIdx.x * blockDim.y + threadIdx.y; }
+// Rows of this thread's row slot: the first, then x_row_step() further down, while
+// >= 0.  The row passes walk the array from its end: the y passes before and after
+// them walk it from its start, so a row pass first meets the planes the y pass wrote
+// last, and leaves last those the next y pass reads first, while they are in L2
+// (256^3 FP32, 128 MB of psi against 126 MB of L2).
+__device__ __forceinline__ long x_row0(long rows) { return rows - 1 - ((long)blockIdx.x * blockDim.y + threadIdx.y); }
 __device__ __forceinline__ long x_row_step() { return (long)gridDim.x * blockDim.y; }
 
 // cp.async 16-byte copy global -> shared (no register round trip) and its groups
@@ -337,7 +341,7 @@ __global__ void __launch_bounds__(256, 3) k_x_fwd(XArgs<R> a) {
     C* sm = x_setup<N, R>(a, smem_raw, tb);
     const int t = threadIdx.x;
     RowAcc<C> acc{sm, warp_lanes_mask()};
-    for (long row = x_row0(); row < a.rows; row += x_row_step()) {
+    for (long row = x_row0(a.rows); row >= 0; row -= x_row_step()) {
         acc.sync();  // this slot's previous row is done with the buffer
         const C* src = a.in + row * N;
         C v[E];
@@ -383,7 +387,7 @@ __global__ void __launch_bounds__(256, 2) k_x_energy(XArgs<R> a, double* part) {
         vrho += (double)v * r;
         vmax = fmax_nan(vmax, fabs((double)v));
     };
-    for (long row = x_row0(); row < a.rows; row += x_row_step()) {
+    for (long row = x_row0(a.rows); row >= 0; row -= x_row_step()) {
         acc.sync();  // this slot's previous row is done with the buffer
         const C* src = a.in + row * N;
         const R* pot = a.Vin + row * N;
@@ -487,8 +491,8 @@ __global__ void __launch_bounds__(256, 2) k_x_inv(XArgs<R> a) {
             cp_async_commit();
         }
     };
-    if (STAGE && x_row0() < a.rows) prefetch(x_row0());
-    for (long row = x_row0(); row < a.rows; row += x_row_step()) {
+    if (STAGE && x_row0(a.rows) >= 0) prefetch(x_row0(a.rows));
+    for (long row = x_row0(a.rows); row >= 0; row -= x_row_step()) {
         acc.sync();
         C v[E];
         if constexpr (STAGE) {
@@ -498,8 +502,8 @@ __global__ void __launch_bounds__(256, 2) k_x_inv(XArgs<R> a) {
             for (int e = 0; e < E; ++e) v[e] = stg[out_pos<N, E>(e, t)];
             // every lane has its values: fetch the next row
             acc.sync();
-            const long nrow = row + x_row_step();
-            if (nrow < a.rows) prefetch(nrow);
+            const long nrow = row - x_row_step();
+            if (nrow >= 0) prefetch(nrow);
         } else {
             const C* src = a.in + row * N;
 #pragma unroll
@@ -563,7 +567,7 @@ __global__ void __launch_bounds__(256, 3) k_x_r2c(XArgs<R> a) {
     const int t = threadIdx.x;
     RowAcc<C> acc{sm, warp_lanes_mask()};
     const R pr = (R)a.pref, rm = (R)a.rho_mean;
-    for (long row = x_row0(); row < a.rows; row += x_row_step()) {
+    for (long row = x_row0(a.rows); row >= 0; row -= x_row_step()) {
         acc.sync();
         C z[EH];
 #pragma unroll
@@ -630,8 +634,8 @@ __global__ void __launch_bounds__(256, 2) k_x_c2r(XArgs<R> a) {
             cp_async_commit();
         }
     };
-    if (x_row0() < a.rows) prefetch(x_row0());
-    for (long row = x_row0(); row < a.rows; row += x_row_step()) {
+    if (x_row0(a.rows) >= 0) prefetch(x_row0(a.rows));
+    for (long row = x_row0(a.rows); row >= 0; row -= x_row_step()) {
         acc.sync();
         if constexpr (STAGE) {
             cp_async_wait_all();
@@ -680,8 +684,8 @@ __global__ void __launch_bounds__(256, 2) k_x_c2r(XArgs<R> a) {
             if constexpr (STAGE) {
                 // every lane is done with the staged row: fetch the next one
                 acc.sync();
-                const long nrow = row + x_row_step();
-                if (nrow < a.rows) prefetch(nrow);
+                const long nrow = row - x_row_step();
+                if (nrow >= 0) prefetch(nrow);
             }
             if constexpr (FLAGS & XC_WRITE_PSI) {
 #pragma unroll

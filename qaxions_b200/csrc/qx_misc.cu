@@ -5,6 +5,7 @@
 #include <string>
 
 #include "qx_kernels.cuh"
+#include "qx_launch.cuh"
 #include "qx_misc.hpp"
 #include "qx_philox.h"
 
@@ -82,6 +83,7 @@ __global__ void __launch_bounds__(kRedThreads) k_reduce(int kind, const cx_t<R>*
                                                         double* partial) {
     __shared__ double red[32];
     double a0 = 0.0, a1 = 0.0;
+    pdl_wait();
     for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < S; i += (long)gridDim.x * blockDim.x) {
         if (kind == RED_RHO) {
             const cx_t<R> p = psi[i];
@@ -103,16 +105,15 @@ __global__ void __launch_bounds__(kRedThreads) k_reduce(int kind, const cx_t<R>*
         partial[blockIdx.x] = s0;
         partial[gridDim.x + blockIdx.x] = s1;
     }
+    pdl_launch();
 }
 
-// one warp (launched <<<1, 32>>>) folds the per-block partials
+// two warps (launched <<<1, 64>>>) fold the per-block partials: sums and maxima
 __global__ void k_fold(const double* partial, int n, double* out) {
-    const double s = warp_fold<0>(partial, n);
-    const double m = warp_fold<1>(partial + n, n);
-    if (threadIdx.x == 0) {
-        out[0] = s;
-        out[1] = m;
-    }
+    pdl_wait();
+    const bool mx = threadIdx.x >= 32;
+    const double v = mx ? warp_fold<1>(partial + n, n) : warp_fold<0>(partial, n);
+    if ((threadIdx.x & 31) == 0) out[mx ? 1 : 0] = v;
 }
 
 // The diagnostics' partials (Ops::energy) folded in a fixed order, one warp per
@@ -121,6 +122,7 @@ __global__ void k_fold(const double* partial, int n, double* out) {
 __global__ void k_fold_energy(const double* part, long cap, long n0, long n1, long n2, double* out) {
     const int w = threadIdx.x >> 5;
     double v;
+    pdl_wait();
     if (w < 5) v = (w & 1) ? warp_fold<1>(part + w * n0, n0) : warp_fold<0>(part + w * n0, n0);
     else v = warp_fold<0>(part + w * cap, w == 5 ? n1 : n2);
     if ((threadIdx.x & 31) == 0) out[w] = v;
@@ -379,14 +381,11 @@ void Misc<R>::rho_to_V(const C* psi, R* V, long S, cudaStream_t st) {
 }
 template <typename R>
 void Misc<R>::reduce(int kind, const C* psi, const R* V, long S, double* partial, double* out, cudaStream_t st) {
-    k_reduce<R><<<kRedBlocks, kRedThreads, 0, st>>>(kind, psi, V, S, partial);
-    QX_CHECK_LAUNCH();
-    k_fold<<<1, 32, 0, st>>>(partial, kRedBlocks, out);
-    QX_CHECK_LAUNCH();
+    launch_dep(k_reduce<R>, dim3(kRedBlocks), dim3(kRedThreads), 0, st, kind, psi, V, S, partial);
+    launch_dep(k_fold, dim3(1), dim3(64), 0, st, partial, kRedBlocks, out);
 }
 void fold_energy(const double* part, long cap, const long (&n)[3], double* out, cudaStream_t st) {
-    k_fold_energy<<<1, 7 * 32, 0, st>>>(part, cap, n[0], n[1], n[2], out);
-    QX_CHECK_LAUNCH();
+    launch_dep(k_fold_energy, dim3(1), dim3(7 * 32), 0, st, part, cap, n[0], n[1], n[2], out);
 }
 template <typename R>
 void Misc<R>::poisson_packed(C* vh, int dim, int N, double pc, double g0, cudaStream_t st) {

@@ -29,7 +29,8 @@ template <typename R> struct Misc {
     static void kick(C* psi, const R* V, double dt, long S, cudaStream_t st);
     // V <- |psi|^2   (Field::computeEnergy, src/field.cxx:205-211)
     static void rho_to_V(const C* psi, R* V, long S, cudaStream_t st);
-    // reductions; partial must hold 2*kRedBlocks doubles, out 2 doubles
+    // reductions; partial must hold 2*kRedBlocks doubles, out 2 doubles (device memory
+    // or host memory mapped into the device)
     static void reduce(int kind, const C* psi, const R* V, long S, double* partial, double* out, cudaStream_t st);
     // Poisson multiplier on a fully transformed packed half spectrum
     // (Field::Poisson, src/field.cxx:230-291)
