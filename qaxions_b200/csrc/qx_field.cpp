@@ -496,10 +496,13 @@ class FieldT final : public Field {
 
     // ---- pass sequences ----
     void y_fwd(C* a, int X) {
-        if (g_.dim == 3) Ops<R>::y_pass(g_.N, g_.B * g_.N, sp(a, X), -1, tune_, st_);
+        y_pass(a, X, -1);
     }
-    void y_inv(C* a, int X) {
-        if (g_.dim == 3) Ops<R>::y_pass(g_.N, g_.B * g_.N, sp(a, X), +1, tune_, st_);
+    void y_inv(C* a, int X) { y_pass(a, X, +1); }
+    void y_pass(C* a, int X, int sign) {
+        if (g_.dim != 3) return;
+        if (direct_on() && Plane<R>::ycol(g_.N, X, sign)) Plane<R>::y_pass(g_.N, g_.B * g_.N, sp(a, X), sign, st_);
+        else Ops<R>::y_pass(g_.N, g_.B * g_.N, sp(a, X), sign, tune_, st_);
     }
     // drift factor tables A(nx, ny), B(nz)/S for time step dt (recomputed only
     // when dt changes; capture_body computes them before a capture begins)
@@ -521,6 +524,7 @@ class FieldT final : public Field {
     }
     // the drift and Poisson passes along the last axis: the direct-load column
     // kernels where the grid has them, else the tile ring
+    bool direct_on() const { return tune_.tma && tune_.plan == 0 && tune_.wp == 0 && planes_; }
     bool col_on() const { return tune_.tma && tune_.plan == 0 && planes_ && Plane<R>::col(g_.N, g_.dim); }
     void last_axis(const typename Ops<R>::SP& s, int op) {
         if (col_on()) Plane<R>::col_pass(g_.N, s, op, st_);

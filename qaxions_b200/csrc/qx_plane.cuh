@@ -445,14 +445,16 @@ template <typename P> struct ColTileAcc {
     __device__ __forceinline__ void sync() const { named_barrier(1, nt); }
 };
 
-template <int N, typename R, int OP, int UX, bool D3>
+// OP_FWD / OP_INV (D3 = false, o = plane): the y transforms of a 3D array whose
+// planes do not fit (FP64 128^3), double-float twiddles when DFT.
+template <int N, typename R, int OP, int UX, bool D3, bool DFT = (OP == OP_DRIFT)>
 __global__ void __launch_bounds__((ColGeo<N, R, UX>::NT + (OP == OP_POISSON && D3 ? ColGeo<N, R, UX>::TX : 0)))
     k_col(SArgs<R> s, const double2* axy) {
     using G = ColGeo<N, R, UX>;
     using C = typename G::C;
     using P = typename G::P;
     constexpr int E = G::E, PW = G::PW;
-    constexpr bool DF = OP == OP_DRIFT;
+    constexpr bool DF = DFT;
     constexpr bool EXTRA = OP == OP_POISSON && D3;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     C* tws = reinterpret_cast<C*>(smem_raw);
@@ -485,8 +487,23 @@ __global__ void __launch_bounds__((ColGeo<N, R, UX>::NT + (OP == OP_POISSON && D
     const long pstride = D3 ? (long)N * s.X : (long)s.X;
     C* base = s.a + (D3 ? (long)(o / N) * N * N * s.X + (long)y * s.X : (long)o * N * s.X) + x0;
     P v[E];
+    ColTileAcc<P> acc{extra ? tile + (size_t)G::prow(N) * UX : tile + u, extra ? 1 : UX, extra || UX != 8, nt};
+    if constexpr (OP == OP_INV) {
+#pragma unroll
+        for (int e = 0; e < E; ++e) v[e] = *reinterpret_cast<const P*>(base + out_pos<N, E>(e, t) * pstride);
+        ifft_pencil_rev<N, E>(v, acc, t, tw_src<DF>(tws, tws_lo));
+#pragma unroll
+        for (int e = 0; e < E; ++e) *reinterpret_cast<P*>(base + in_pos<N, E, 0>(e, t) * pstride) = v[e];
+        return;
+    }
 #pragma unroll
     for (int e = 0; e < E; ++e) v[e] = *reinterpret_cast<const P*>(base + in_pos<N, E, 0>(e, t) * pstride);
+    if constexpr (OP == OP_FWD) {
+        fft_pencil<N, E, -1>(v, acc, t, tw_src<DF>(tws, tws_lo));
+#pragma unroll
+        for (int e = 0; e < E; ++e) *reinterpret_cast<P*>(base + out_pos<N, E>(e, t) * pstride) = v[e];
+        return;
+    }
     double2 A[PW];
     if constexpr (OP == OP_DRIFT) {
         const double2* gbz = axy + (D3 ? (long)N * N : (long)N);
@@ -494,7 +511,6 @@ __global__ void __launch_bounds__((ColGeo<N, R, UX>::NT + (OP == OP_POISSON && D
 #pragma unroll
         for (int h = 0; h < PW; ++h) A[h] = axy[(D3 ? (long)y * N : 0L) + x0 + h];
     }
-    ColTileAcc<P> acc{extra ? tile + (size_t)G::prow(N) * UX : tile + u, extra ? 1 : UX, extra || UX != 8, nt};
     fft_pencil<N, E, -1>(v, acc, t, tw_src<DF>(tws, tws_lo));
     if constexpr (OP == OP_DRIFT) {
         // the forward transform's exchanges have synchronised the block since bz was written

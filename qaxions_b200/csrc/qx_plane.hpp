@@ -27,6 +27,9 @@ template <typename R> struct Plane {
     // vh (transformed along x and y) -> V, with the flags of Ops::x_c2r; with
     // C2R_FWD psi goes on to psi^_xy
     static void c2r(int N, const XP& a, int flags, cudaStream_t st);
+    // y transform (sign -1 forward, +1 inverse) of [planes][N][X], where the grid has one
+    static bool ycol(int N, int X, int sign);
+    static void y_pass(int N, int planes, const SP& a, int sign, cudaStream_t st);
     // last-axis drift or Poisson pass (OP_DRIFT on psi, OP_POISSON on vh, column 0 included)
     static void col_pass(int N, const SP& a, int op, cudaStream_t st);
 };

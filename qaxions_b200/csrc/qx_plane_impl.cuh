@@ -97,6 +97,45 @@ static void launch_col(const typename Ops<R>::SP& a, int op, cudaStream_t st) {
     }
 }
 
+template <int NN, typename R>
+static void launch_ycol(const typename Ops<R>::SP& a, int planes, int sign, cudaStream_t st) {
+    using G = ColGeo<NN, R, 8>;
+    SArgs<R> s = to_s<R>(a);
+    const unsigned grid = (unsigned)(a.X / (8 * G::PW)) * (unsigned)planes;
+    const bool df = sizeof(R) == 4 && a.tw_lo != nullptr;
+    auto go = [&](auto kern) {
+        const size_t smem = G::smem(OP_FWD, false);
+        set_smem(kern, smem);
+        launch_dep(kern, dim3(grid), dim3(G::NT), smem, st, s, (const double2*)nullptr);
+    };
+    if (sign < 0) {
+        if (df) go(k_col<NN, R, OP_FWD, 8, false, true>);
+        else go(k_col<NN, R, OP_FWD, 8, false, false>);
+    } else {
+        if (df) go(k_col<NN, R, OP_INV, 8, false, true>);
+        else go(k_col<NN, R, OP_INV, 8, false, false>);
+    }
+}
+
+// FP64 128^3, whose planes do not fit: all y passes (step 106 -> 101 us).  256^3 FP32,
+// 128 + 64 MB in and out of L2: psi forward 54 -> 50 us and the half spectrum 31 / 29
+// -> 28 / 27; psi inverse is faster from the ring (54 against 59), and so are the
+// last-axis passes (z drift 99 against 107); 256^3 FP64 gains nowhere (z Poisson 97
+// against 143).
+template <typename R> bool Plane<R>::ycol(int N, int X, int sign) {
+    if (N == 128) return sizeof(R) == 8;
+    return N == 256 && sizeof(R) == 4 && (X < N || sign < 0);
+}
+
+template <typename R> void Plane<R>::y_pass(int N, int planes, const SP& a, int sign, cudaStream_t st) {
+    if constexpr (sizeof(R) == 8) {
+        if (N == 128) return launch_ycol<128, R>(a, planes, sign, st);
+    } else {
+        if (N == 256) return launch_ycol<256, R>(a, planes, sign, st);
+    }
+    throw std::logic_error("y column pass: not compiled");
+}
+
 template <typename R> void Plane<R>::col_pass(int N, const SP& a, int op, cudaStream_t st) {
     if ((op != OP_DRIFT && op != OP_POISSON) || !col(N, a.dim)) throw std::logic_error("column pass: not compiled");
     if (a.dim == 3) {
