@@ -615,18 +615,26 @@ __global__ void __launch_bounds__(256) k_wgrad(const __nv_bfloat16* __restrict__
 //      start address.
 //   B  dZ stored [row][chunk][x][8 channels]: LBO = NC / 8 * 128 B, SBO = 128 B.
 // Per 8 x 8 x 4 brick (K = 256 sites) one thread issues 16 MMAs (M = 128, N = NC, K
-// = 16) into each of 9 accumulators of NC tensor-memory columns, which add up over
-// all bricks of the block.  Bricks arrive by cp.async in a ring of three: while
-// the MMAs of brick k run, brick k + 1 is there and k + 2 is under way.  Bound by the
-// MMAs' reads of A (82 cycles for 4 KB).  Building each offset group's shifted
-// operand through registers instead was bound by that copy: at 128^3, us, 32 -> 32
-// layer 1442 -> 344, 4 -> 32 876 -> 303, 32 -> 2 1488 -> 318.  Waits are bounded;
+// = 16) into each of 9 accumulators of NC tensor-memory columns (6 for the input
+// layer), which add up over all bricks of the block.  Bricks arrive by cp.async in
+// a ring of three: while the MMAs of brick k run, brick k + 1 is there and k + 2 is
+// under way, copied by the other seven warps.  Bound by the MMAs (about 55 cycles
+// each for M = 128, N = 32).  Building each offset group's shifted operand through
+// registers instead was bound by that copy: at 128^3, us, 32 -> 32 layer 1442 -> 288,
+// 4 -> 32 876 -> 140, 32 -> 2 1488 -> 254.  Waits are bounded;
 // tensor memory is freed on every path.  partial: [gridDim.x][27 * cin * cout].
 namespace wtc {
 constexpr int STAGES = 3;
 constexpr int ROWS = BY * BZ;  // rows of 8 sites in a brick
 template <int CINP, int NC> struct Geo {
-    static constexpr int KC = CINP / 8;                      // 16-byte channel chunks per site
+    static constexpr int KC = CINP == 16 ? 1 : CINP / 8;     // 16-byte channel chunks per site that are used
+    // CINP = 16 is the input layer: its 4 features lie in the first chunk.  With one
+    // chunk per row the 16 M groups are 16 halo rows, and row + HY = 10 is the next
+    // plane's: an MMA covers dy = -1, 0, 1 of dz and of dz + 1, and 6 accumulators
+    // (dz = -1 with 0, dz = 1; three dx) take the place of 9.
+    static constexpr int DZS = KC == 1 ? 2 : 3;   // dz starts
+    static constexpr int NACC = 3 * DZS;          // accumulators
+    static constexpr int BPS = KC == 1 ? 2 : 1;   // blocks per SM (shared and tensor memory)
     static constexpr int HALO_BYTES = HZ * HY * KC * HX * 16;  // 38,400 for CINP = 32
     static constexpr int DZ_BYTES = ROWS * (NC / 8) * 128;     // 16,384 for NC = 32
     static constexpr int STAGE_BYTES = HALO_BYTES + DZ_BYTES;
@@ -634,16 +642,17 @@ template <int CINP, int NC> struct Geo {
     static constexpr size_t SMEM = (size_t)STAGES * STAGE_BYTES + 16 * HX * 16 + 128;
     static constexpr uint32_t LBO_A = KC * HX * 16, SBO_A = HX * 16;
     static constexpr uint32_t LBO_B = NC / 8 * 128, SBO_B = 128;
-    static constexpr uint32_t TMEM_COLS = 9 * NC <= 256 ? 256 : 512;
+    static constexpr uint32_t TMEM_COLS = NACC * NC <= 256 ? 256 : 512;
     // D FP32, A and B BF16, both MN-major (bits 15, 16), N >> 3, M >> 4
     static constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) |
                                       ((uint32_t)(NC >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
     static_assert(HALO_BYTES % 128 == 0 && DZ_BYTES % 128 == 0, "operand alignment");
+    static_assert(HY == 10, "the next plane's rows in the M groups");
 };
 }  // namespace wtc
 
 template <int CINP, int NC>
-__global__ void __launch_bounds__(256, 1) k_wgrad_tc(const __nv_bfloat16* __restrict__ A,
+__global__ void __launch_bounds__(256, (wtc::Geo<CINP, NC>::BPS)) k_wgrad_tc(const __nv_bfloat16* __restrict__ A,
                                                      const __nv_bfloat16* __restrict__ dZ, int N, int cin, int cout,
                                                      float* partial, int* err) {
     using G = wtc::Geo<CINP, NC>;
@@ -677,21 +686,23 @@ __global__ void __launch_bounds__(256, 1) k_wgrad_tc(const __nv_bfloat16* __rest
     const int nbx = N / BX, nby = N / BY, nbz = N / BZ;
     const int nbricks = nbx * nby * nbz;
     const int mine = blockIdx.x < nbricks ? (nbricks - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
-    // copy the k-th brick of this block into its stage (one cp.async group, empty past the end)
+    // copy the k-th brick of this block into its stage (one cp.async group, empty past
+    // the end); warp 0 only issues MMAs, so that they follow one another without a gap
+    const int lt = tid - 32, lstep = blockDim.x - 32;
     auto load = [&](int k) {
-        if (k < mine) {
+        if (k < mine && lt >= 0) {
             const int br = blockIdx.x + k * gridDim.x;
             const int bxi = br % nbx, byi = (br / nbx) % nby, bzi = br / (nbx * nby);
             const int x0 = bxi * BX, y0 = byi * BY, z0 = bzi * BZ;
             const uint32_t st = smem_addr(base) + (uint32_t)((k % wtc::STAGES) * G::STAGE_BYTES);
-            for (int i = tid; i < HZ * HY * KC * HX; i += blockDim.x) {
+            for (int i = lt; i < HZ * HY * KC * HX; i += lstep) {
                 const int hx = i % HX, ch = (i / HX) % KC, hy = (i / (HX * KC)) % HY, hz = i / (HX * KC * HY);
                 const long gs = ((long)wrapi(z0 + hz - 1, N) * N + wrapi(y0 + hy - 1, N)) * N + wrapi(x0 + hx - 1, N);
                 asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(st + (uint32_t)i * 16),
                              "l"(A + gs * CINP + ch * 8)
                              : "memory");
             }
-            for (int i = tid; i < wtc::ROWS * (NC / 8) * 8; i += blockDim.x) {  // [row][x][chunk] reads whole lines
+            for (int i = lt; i < wtc::ROWS * (NC / 8) * 8; i += lstep) {  // [row][x][chunk] reads whole lines
                 const int ch = i % (NC / 8), x = (i / (NC / 8)) % 8, r = i / NC;
                 const long gs = ((long)(z0 + r / BY) * N + (y0 + r % BY)) * N + (x0 + x);
                 asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(st + (uint32_t)(G::HALO_BYTES +
@@ -719,15 +730,19 @@ __global__ void __launch_bounds__(256, 1) k_wgrad_tc(const __nv_bfloat16* __rest
         }
         if (tid == 0) {
             fence_after();
-            const uint32_t h0 = smem_addr(base) + (uint32_t)((k % wtc::STAGES) * G::STAGE_BYTES), d0 = h0 + G::HALO_BYTES;
+            const uint32_t h0 = smem_addr(base) + (uint32_t)((k % wtc::STAGES) * G::STAGE_BYTES);
+            const uint64_t a0 = smem_desc(h0, G::LBO_A, G::SBO_A);
+            const uint64_t b0 = smem_desc(h0 + G::HALO_BYTES, G::LBO_B, G::SBO_B);
 #pragma unroll 1
             for (int r = 0; r < wtc::ROWS; r += 2) {  // rows y, y + 1 of plane z
                 const int y = r % BY, z = r / BY;
-                const uint64_t bd = smem_desc(d0 + (uint32_t)(r * (NC / 8) * 128), G::LBO_B, G::SBO_B);
+                // address fields advance in 16-byte units
+                const uint64_t ar = a0 + (uint64_t)((z * HY + y) * KC * HX);
+                const uint64_t br = b0 + (uint64_t)(r * (NC / 8) * 8);
 #pragma unroll
-                for (int q = 0; q < 9; ++q) {  // (dz, dx) = (q / 3 - 1, q % 3 - 1); start row dy = -1
-                    const uint32_t ad = h0 + (uint32_t)((((z + q / 3) * HY + y) * KC * HX + q % 3) * 16);
-                    tc::mma<G::IDESC>(tmem + (uint32_t)(q * NC), smem_desc(ad, G::LBO_A, G::SBO_A), bd,
+                for (int q = 0; q < G::NACC; ++q) {  // dz start (q / 3), dx = q % 3 - 1; start row dy = -1
+                    const int zq = G::DZS == 2 ? 2 * (q / 3) : q / 3;
+                    tc::mma<G::IDESC>(tmem + (uint32_t)(q * NC), ar + (uint64_t)(zq * HY * KC * HX + q % 3), br,
                                       (k > 0 || r > 0) ? 1u : 0u);
                 }
             }
@@ -746,16 +761,19 @@ __global__ void __launch_bounds__(256, 1) k_wgrad_tc(const __nv_bfloat16* __rest
     if (__syncthreads_or(fail)) abort = true;
     const int nw = KOFF * cin * cout;
     float* outp = partial + (long)blockIdx.x * nw;
-    // accumulator row m = channel m % CINP at dy = m / CINP - 1; warps w and w + 4 read
-    // rows 32 (w % 4) .. of accumulators 0, 2, .. and 1, 3, ..
+    // accumulator row m = channel m % (8 KC) of halo row m / (8 KC) after the start
+    // (dy = -1): dy - 1 + row, for one chunk from row HY on of the next plane; warps w
+    // and w + 4 read rows 32 (w % 4) .. of accumulators 0, 2, .. and 1, 3, ..
     if (!abort) {
         const int m = 32 * (warp & 3) + lane;
-        const int ci = m % CINP, dyi = m / CINP;
-        for (int q = warp >> 2; q < 9; q += 2) {
+        const int ci = m % (8 * KC), row = m / (8 * KC);
+        const int plane = KC == 1 ? row / HY : 0, dyi = row - plane * HY;
+        for (int q = warp >> 2; q < G::NACC; q += 2) {
             float v[32];
             tc::tmem_ld32(tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(q * NC), v);
-            const int o = (q / 3) * 9 + dyi * 3 + q % 3;
-            if (dyi < 3 && ci < cin)
+            const int dzi = (G::DZS == 2 ? 2 * (q / 3) : q / 3) + plane;
+            const int o = dzi * 9 + dyi * 3 + q % 3;
+            if (dyi < 3 && dzi < 3 && ci < cin)
 #pragma unroll
                 for (int co = 0; co < NC; ++co)
                     if (co < cout) outp[(o * cin + ci) * cout + co] = mine > 0 ? v[co] : 0.f;
@@ -1227,14 +1245,14 @@ class Corrector {
         k_fold<<<1, 256, 0, st_>>>(bpart_.as<float>(), blocks, L.cout, L.gb.as<float>());
     }
     // weight gradient of layer L from its input A and dZ: on the tensor cores from
-    // the BF16 dZb [S][NC] (one block per SM; the bias gradient of all but the last
+    // the BF16 dZb [S][NC] (as many blocks as fit at once; the bias gradient of all but the last
     // layer comes with back()), or the CUDA-core sums of the FP32 dZ (set_tensor_path(0))
     template <int CINP, int NC>
     void wgrad(const __nv_bfloat16* A, const float* dZ, const __nv_bfloat16* dZb, Layer& L) {
         const int nbricks = (int)(S_ / BSITES);
         const int nw = KOFF * L.cin * L.cout;
         if (use_tc_) {
-            const int nblk = std::min(nbricks, sms());
+            const int nblk = std::min(nbricks, sms() * wtc::Geo<CINP, NC>::BPS);
             part_.alloc(sizeof(float) * (size_t)nblk * nw);
             k_wgrad_tc<CINP, NC><<<nblk, 256, wtc::Geo<CINP, NC>::SMEM, st_>>>(A, dZb, N_, L.cin, L.cout,
                                                                                part_.as<float>(), errb_.as<int>());
