@@ -322,6 +322,51 @@ template <int SIGN, typename C> __device__ __forceinline__ CPair<C> tw_mul(CPair
     return {df_mul(v.a, w, l), df_mul(v.b, w, l)};
 }
 
+// Register slot of the twiddle of butterfly b, input m, stage s of a thread that
+// keeps its own: one set of r - 1 per butterfly column, or one for the stage where
+// every column of the thread has the same (T a multiple of the span).
+template <int L, int E, int s> __host__ __device__ constexpr int tw_slots() {  // slots before stage s
+    if constexpr (s <= 1) return 0;
+    else {
+        constexpr int r = qx_radix(L, s - 1), Ns = qx_span(L, s - 1), T = qx_len(L) / E;
+        return tw_slots<L, E, s - 1>() + (T % Ns == 0 ? 1 : E / r) * (r - 1);
+    }
+}
+template <int L, int E, int s> __host__ __device__ constexpr int tw_slot(int b, int m) {
+    constexpr int r = qx_radix(L, s), Ns = qx_span(L, s), T = qx_len(L) / E;
+    return tw_slots<L, E, s>() + (T % Ns == 0 ? 0 : b) * (r - 1) + m - 1;
+}
+// a thread's own twiddles (hi + lo when DF), read from the tables once
+template <int L, int E, bool DF, typename C> struct TwRegs {
+    static constexpr int NT = tw_slots<L, E, qx_nstages(L)>();
+    C hi[NT];
+    C lo[DF ? NT : 1];
+    template <int s = 1> __device__ __forceinline__ void load(const C* thi, const C* tlo, int t) {
+        if constexpr (s < qx_nstages(L)) {
+            constexpr int r = qx_radix(L, s), Ns = qx_span(L, s), T = qx_len(L) / E;
+#pragma unroll
+            for (int b = 0; b < (T % Ns == 0 ? 1 : E / r); ++b)
+#pragma unroll
+                for (int m = 1; m < r; ++m) {
+                    const int i = qx_tw_index(L, Ns, m, (t + b * T) % Ns);
+                    hi[tw_slot<L, E, s>(b, m)] = thi[i];
+                    if constexpr (DF) lo[tw_slot<L, E, s>(b, m)] = tlo[i];
+                }
+            load<s + 1>(thi, tlo, t);
+        }
+    }
+};
+// the twiddle at table index i or register slot, as a source of its own
+template <typename C> __device__ __forceinline__ const C* tw_at(const C* tw, int i, int) { return tw + i; }
+template <typename C> __device__ __forceinline__ TwPair<C> tw_at(const TwPair<C>& tw, int i, int) {
+    return {tw.hi + i, tw.lo + i};
+}
+template <int L, int E, bool DF, typename C>
+__device__ __forceinline__ auto tw_at(const TwRegs<L, E, DF, C>& tw, int, int slot) {
+    if constexpr (DF) return TwPair<C>{&tw.hi[slot], &tw.lo[slot]};
+    else return static_cast<const C*>(&tw.hi[slot]);
+}
+
 // Position held by v[e] in the OUTPUT order of forward stage s (where stage s
 // writes its results); for the last stage this is out_pos.
 template <int L, int E, int s, int J0 = 0> __device__ __forceinline__ int stage_out_pos(int e, int t) {
@@ -345,7 +390,7 @@ __device__ __forceinline__ void fft_stages(C (&v)[E], Acc& acc, int t, const TW&
             if constexpr (Ns > 1) {
                 const int k = j % Ns;
 #pragma unroll
-                for (int m = 1; m < r; ++m) v[b * r + m] = tw_mul<SIGN>(v[b * r + m], tw, qx_tw_index(L, Ns, m, k));
+                for (int m = 1; m < r; ++m) v[b * r + m] = tw_mul<SIGN>(v[b * r + m], tw_at(tw, qx_tw_index(L, Ns, m, k), tw_slot<L, E, s>(b, m)), 0);
             }
             dft<r, SIGN>(&v[b * r]);
         }
@@ -416,7 +461,7 @@ __device__ __forceinline__ void ifft_rev_stages(C (&v)[E], Acc& acc, int t, cons
         if constexpr (Ns > 1) {
             const int k = stage_j<L, E, s, J0>(b, t) % Ns;
 #pragma unroll
-            for (int m = 1; m < r; ++m) v[b * r + m] = tw_mul<+1>(v[b * r + m], tw, qx_tw_index(L, Ns, m, k));
+            for (int m = 1; m < r; ++m) v[b * r + m] = tw_mul<+1>(v[b * r + m], tw_at(tw, qx_tw_index(L, Ns, m, k), tw_slot<L, E, s>(b, m)), 0);
         }
     }
     if constexpr (s > 0) {

@@ -272,6 +272,16 @@ __global__ void __launch_bounds__((tma_block_threads<N, R, PW, TXF>()), (tma_blo
     }
     __syncthreads();
 
+    // half-spectrum passes at 512 (single twiddles, E = 8): a thread's own twiddles stay in
+    // registers (z Poisson 383 -> 371 us, y inverse 197 -> 186; at 256 they cost a
+    // block's worth of registers: z Poisson 54 -> 60)
+    constexpr bool TWREG = PW == 2 && !DF && TXF == 8 && N == 512 && OP != OP_KIN;
+    TwRegs<NL, E, false, C> twr;
+    if constexpr (TWREG) twr.load(tws, tws_lo, t);
+    auto tw = [&]() -> decltype(auto) {
+        if constexpr (TWREG) return (twr);
+        else return tw_src<DF>(tws, tws_lo);
+    };
     double kin = 0.0;
     int k = 0;
     for (;; ++k) {
@@ -302,11 +312,11 @@ __global__ void __launch_bounds__((tma_block_threads<N, R, PW, TXF>()), (tma_blo
         if constexpr (OP == OP_INV) {
 #pragma unroll
             for (int e = 0; e < E; ++e) v[e] = acc(out_pos<NL, E>(e, t));
-            ifft_pencil_rev<NL, E>(v, acc, t, tw_src<DF>(tws, tws_lo));
+            ifft_pencil_rev<NL, E>(v, acc, t, tw());
         } else {
 #pragma unroll
             for (int e = 0; e < E; ++e) v[e] = acc(in_pos<NL, E, 0>(e, t));
-            fft_pencil<NL, E, -1>(v, acc, t, tw_src<DF>(tws, tws_lo));
+            fft_pencil<NL, E, -1>(v, acc, t, tw());
         }
 
         // |n|^2 contribution of x (and y in 3D) of pencil h
@@ -389,7 +399,7 @@ __global__ void __launch_bounds__((tma_block_threads<N, R, PW, TXF>()), (tma_blo
             }
             // inverse transform: the forward stages undone in reverse order,
             // from the forward output order back to the load order
-            ifft_pencil_rev<NL, E>(v, acc, t, tw_src<DF>(tws, tws_lo));
+            ifft_pencil_rev<NL, E>(v, acc, t, tw());
             if (OP == OP_POISSON && s.col0_external && x0 == 0) {
                 // the stash was written in another order by other threads; a
                 // multi-stage inverse already synchronised the block
@@ -595,6 +605,16 @@ __global__ void __launch_bounds__(kWpThreads * WPP, 1) k_pencil_wp(const __grid_
     }
     __syncthreads();
 
+    // the same for every tile: a thread's twiddles stay in registers where they fit
+    // (512^3, us: FP32 z drift 690 -> 650, y forward 383 -> 360; FP64 z drift 1100 ->
+    // 1075, y forward 766 -> 728); two table loads fewer per value and transform
+    constexpr bool TWREG = OP != OP_POISSON && WPP == 1;
+    TwRegs<NL, E, DF && sizeof(R) == 4, C> twr;
+    if constexpr (TWREG) twr.load(tws, tws_lo, t);
+    auto tw = [&]() -> decltype(auto) {
+        if constexpr (TWREG) return (twr);
+        else return tw_src<DF>(tws, tws_lo);
+    };
     double kin = 0.0;
     int k = 0;
     for (;; ++k) {
@@ -620,11 +640,11 @@ __global__ void __launch_bounds__(kWpThreads * WPP, 1) k_pencil_wp(const __grid_
         if constexpr (OP == OP_INV) {
 #pragma unroll
             for (int e = 0; e < E; ++e) v[e] = io(out_pos<NL, E>(0, t), out_pos<NL, E>(e, 0));
-            ifft_pencil_rev<NL, E>(v, acc, t, tw_src<DF>(tws, tws_lo));
+            ifft_pencil_rev<NL, E>(v, acc, t, tw());
         } else {
 #pragma unroll
             for (int e = 0; e < E; ++e) v[e] = io(t, in_pos<NL, E, 0>(e, 0));
-            fft_pencil<NL, E, -1>(v, acc, t, tw_src<DF>(tws, tws_lo));
+            fft_pencil<NL, E, -1>(v, acc, t, tw());
         }
         auto mxy_of = [&](int h) {
             const int x = xb + h;
@@ -700,7 +720,7 @@ __global__ void __launch_bounds__(kWpThreads * WPP, 1) k_pencil_wp(const __grid_
                     }
                 }
             }
-            ifft_pencil_rev<NL, E>(v, acc, t, tw_src<DF>(tws, tws_lo));
+            ifft_pencil_rev<NL, E>(v, acc, t, tw());
             if (c0ext) {
                 // the stash was written by other threads of this pencil pair in another
                 // order; the inverse's exchanges synchronised the pair since
