@@ -89,7 +89,7 @@ int qx_drift_update(qx_field_t *h);
 int qx_propagate(qx_field_t *h);
 /* The KDK time loop of main() (src/main.cxx:64-85) with measurements off:
  * updatePotential, half_kick, nsteps x (drift_update, full_kick but the last),
- * half_kick -- fused passes, loop body replayed from a CUDA graph. */
+ * half_kick -- fused passes, loop bodies replayed from a CUDA graph. */
 int qx_step(qx_field_t *h, int nsteps);
 
 /* Field::Vmax / rhomax / time / a / curr (src/field.h:56-62) */
@@ -182,7 +182,7 @@ int qx_set_tune(qx_field_t *h, int x_rows, int y_tx, int la_tx, int tma, int nbu
  * order, for grids whose default plan mixes radix sizes (N = 64, 96, 128,
  * 256); elsewhere plan 1 runs as plan 0.  Results agree to round-off. */
 int qx_set_plan(qx_field_t *h, int plan);
-/* Pencil-to-thread mapping of the FP32 strided passes at N = 256 and 512 (no
+/* Pencil-to-thread mapping of the strided passes at N = 256 and 512 (no
  * counterpart in the reference): 8-column tiles with a pencil pair per 64
  * (N = 512) threads and block-wide stage exchanges, or 16-column swizzled tiles
  * with one warp per pencil pair, warp-local exchanges and one block barrier
@@ -190,8 +190,10 @@ int qx_set_plan(qx_field_t *h, int plan);
  * the wave-function arrays; 2: the warp passes everywhere; 3 / 4 (N = 512):
  * as 1, with each pencil pair split over two warps (16 warps per SM, pair
  * barriers) in the drift pass / in every wave-function pass, bit for bit the
- * one-warp form.  The 3D 512^3 default is 3 (measured fastest).  Results
- * agree to round-off. */
+ * one-warp form.  FP64 at N = 512: any non-zero value runs the wave-function
+ * passes with one warp per pencil in 8-column tiles and the Poisson pass with
+ * two.  The 3D 512^3 default is 1 (measured fastest).  Results agree to
+ * round-off. */
 int qx_set_pencil_warp(qx_field_t *h, int on);
 /* the launch geometry in use: out[10] = {x_rows, y_tx, la_tx, tma, nbuf, pw,
  * plan, chain, pencil_warp, from_cache}, and out[10] = row_stage when n >= 11;
