@@ -524,6 +524,7 @@ class FieldT final : public Field {
     }
     // the drift and Poisson passes along the last axis: the direct-load column
     // kernels where the grid has them, else the tile ring
+    // direct-load y passes (Plane::ycol) unless a tile geometry was asked for
     bool direct_on() const { return tune_.tma && tune_.plan == 0 && tune_.wp == 0 && planes_; }
     bool col_on() const { return tune_.tma && tune_.plan == 0 && planes_ && Plane<R>::col(g_.N, g_.dim); }
     void last_axis(const typename Ops<R>::SP& s, int op) {
