@@ -877,7 +877,9 @@ class FieldT final : public Field {
                     body(ds_, ds_, pref_eff(), true);
                     updateTime();
                 } else {  // all steps up to the next measured or last one
-                    const long stop = next < ml.size() ? std::min<long>(ml[next], nsteps - 1) : nsteps - 1;
+                    // (an entry behind idx, repeated after it was measured, is never met)
+                    const bool ahead = next < ml.size() && ml[next] > (long)idx;
+                    const long stop = ahead ? std::min<long>(ml[next], nsteps - 1) : nsteps - 1;
                     bodies((int)(stop - idx));
                     for (long i = idx; i < stop; ++i) updateTime();
                     idx = (int)stop - 1;
