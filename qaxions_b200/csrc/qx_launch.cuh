@@ -17,11 +17,19 @@ namespace qx {
         if (e_ != cudaSuccess) throw std::runtime_error(std::string("kernel launch: ") + cudaGetErrorString(e_)); \
     } while (0)
 
+// Report a refused call whose status was returned to us.  The runtime also keeps it
+// as its last error, which the next launch check of this thread would take for its
+// own: clear it.
+[[noreturn]] static inline void throw_refused(const char* what, cudaError_t e) {
+    cudaGetLastError();
+    throw std::runtime_error(what + std::string(cudaGetErrorString(e)));
+}
+
 template <typename K>
 static void set_smem(K kernel, size_t bytes) {
     if (bytes > 40 * 1024) {  // (48 KB without the attribute, less the kernel's static arrays)
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-        if (e != cudaSuccess) throw std::runtime_error(std::string("smem attribute: ") + cudaGetErrorString(e));
+        if (e != cudaSuccess) throw_refused("smem attribute: ", e);
     }
 }
 
@@ -43,7 +51,7 @@ static void launch_dep(void (*kern)(KA...), dim3 grid, dim3 block, size_t smem, 
     cfg.attrs = at;
     cfg.numAttrs = 1;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, static_cast<KA>(args)...);
-    if (e != cudaSuccess) throw std::runtime_error(std::string("kernel launch: ") + cudaGetErrorString(e));
+    if (e != cudaSuccess) throw_refused("kernel launch: ", e);
 }
 
 template <typename R> static XArgs<R> to_x(const typename Ops<R>::XP& a) {

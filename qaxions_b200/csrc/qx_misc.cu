@@ -400,7 +400,7 @@ static void launch_spec_bin(const cx_t<R>* vh, long rows, int dim, const int* T,
     const size_t smem = (size_t)(threads / 32) * nbins * (sizeof(double) + sizeof(long long));
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(k_spec_bin<N, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) throw std::runtime_error(std::string("smem attribute: ") + cudaGetErrorString(e));
+        if (e != cudaSuccess) throw_refused("smem attribute: ", e);
     }
     // the guess of spec_bin_of: shells sqrt(M), nbins sqrt(M) / nmax, nbins log(M) / (2 log(nmax))
     const float nmax = (float)(N / 2);
