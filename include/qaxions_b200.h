@@ -175,12 +175,16 @@ int qx_profile_step(qx_field_t *h, int nsteps, int max_entries, char *names, dou
 /* launch geometry overrides (0 = default): rows per x-pass block, tile columns
  * of y / last-axis passes, strided-pass kernel family (1 = TMA-fed persistent,
  * 0 = direct loads; -1 = keep), TMA ring depth, pencils per thread of the TMA
- * passes (1 or 2; 0 = default: 2 in the FP32 form, FP64 always 1) */
+ * passes (1 or 2; 0 = default: 2 in the FP32 form, FP64 always 1).  The grids with
+ * plane-resident or direct-load passes (3D N = 32 ... 128, 2D N = 64 ... 512, FP32
+ * 256^3) run them while every override that describes another form is 0: ring
+ * depth, pencils per thread, tile columns of the pass, and x-pass rows for the
+ * plane-resident ones. */
 int qx_set_tune(qx_field_t *h, int x_rows, int y_tx, int la_tx, int tma, int nbuf, int pw);
 /* Radix plan of the TMA strided (y / last-axis) passes, no counterpart in the
  * reference (FFTW plans its own): 0 default, 1 the same radices in reverse
- * order, for grids whose default plan mixes radix sizes (N = 64, 96, 128,
- * 256); elsewhere plan 1 runs as plan 0.  Results agree to round-off. */
+ * order, for grids whose default plan mixes radix sizes (N = 96, 128, 256);
+ * elsewhere plan 1 runs as plan 0.  Results agree to round-off. */
 int qx_set_plan(qx_field_t *h, int plan);
 /* Pencil-to-thread mapping of the strided passes at N = 256 and 512 (no
  * counterpart in the reference): 8-column tiles with a pencil pair per 64

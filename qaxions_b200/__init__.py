@@ -425,12 +425,14 @@ class Field:
     def set_tune(self, x_rows: int = 0, y_tx: int = 0, la_tx: int = 0, tma: int = -1, nbuf: int = 0, pw: int = 0):
         """Launch geometry overrides (0 = default); tma 1/0 selects the TMA-fed
         persistent or the direct-load strided kernels (-1 keeps the current);
-        pw: pencils per thread of the TMA passes (0 default, 1 or 2)."""
+        pw: pencils per thread of the TMA passes (0 default, 1 or 2).  Grids
+        with plane-resident or direct-load passes run them while no override
+        asks for the ring or the row blocks."""
         self._c("qx_set_tune", x_rows, y_tx, la_tx, tma, nbuf, pw)
 
     def set_plan(self, plan: int):
         """Radix plan of the strided passes: 0 default, 1 reversed radix order
-        (grids N = 64, 96, 128, 256; elsewhere it runs as 0)."""
+        (grids N = 96, 128, 256; elsewhere it runs as 0)."""
         self._c("qx_set_plan", int(plan))
 
     def get_tune(self) -> dict:

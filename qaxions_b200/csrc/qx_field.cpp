@@ -542,11 +542,21 @@ class FieldT final : public Field {
         s.axy = ensure_axy(dt);
         last_axis(s, OP_DRIFT);
     }
-    // the drift and Poisson passes along the last axis: the direct-load column
-    // kernels where the grid has them, else the tile ring
-    // direct-load y passes (Plane::ycol) unless a tile geometry was asked for
-    bool direct_on() const { return tune_.tma && tune_.plan == 0 && tune_.wp == 0 && planes_; }
-    bool col_on() const { return tune_.tma && tune_.plan == 0 && planes_ && Plane<R>::col(g_.N, g_.dim); }
+    // The direct-load and plane-resident passes take no geometry: a setting that
+    // describes the tile ring or the row blocks (set_tune, set_plan and
+    // set_pencil_warp where the grid has the form, the autotuner's choice) runs those.
+    bool ring_asked() const {
+        const bool plan = tune_.plan != 0 && tw_.N_p1;
+        const bool wp = tune_.wp != 0 && (g_.N == 512 || (g_.N == 256 && sizeof(R) == 4));
+        return !tune_.tma || tune_.nbuf || tune_.pw || plan || wp || !planes_;
+    }
+    // direct-load y passes, where Plane::ycol has them
+    bool direct_on() const { return !ring_asked() && tune_.y_tx == 0; }
+    // direct-load drift and Poisson passes along the last axis
+    bool col_on() const {
+        const int tx = g_.dim == 2 && g_.B > 1 ? tune_.y_tx : tune_.la_tx;  // as launch_tma_e takes it
+        return !ring_asked() && tx == 0 && Plane<R>::col(g_.N, g_.dim);
+    }
     void last_axis(const typename Ops<R>::SP& s, int op) {
         if (col_on()) Plane<R>::col_pass(g_.N, s, op, st_);
         else Ops<R>::la_pass(g_.N, s, op, tune_, st_);
@@ -555,7 +565,9 @@ class FieldT final : public Field {
     // a plane (and the pointwise work between them) in one launch; between the
     // launches of the merged loop psi is then transformed along x and y (psi^_xy)
     // instead of along x only
-    bool planes_on() const { return g_.dim == 3 && Plane<R>::xy(g_.N) && col_on() && !chain_on(); }
+    bool planes_on() const {
+        return g_.dim == 3 && Plane<R>::xy(g_.N) && col_on() && direct_on() && tune_.x_rows == 0 && !chain_on();
+    }
     void set_planes(bool on) override {
         if (on != planes_) invalidate_graph();
         planes_ = on;

@@ -32,7 +32,7 @@ struct Tune {
                       // wave-function pass, 0 none.  FP64, N = 512: any non-zero value, the
                       // wave-function passes and (two warps per pencil) the Poisson pass
     int plan = 0;     // radix plan of the TMA strided passes: 0 default order, 1 reversed
-                      // (grids whose plan has radices of different sizes: 64, 96, 128, 256)
+                      // (grids whose plan has radices of different sizes: 96, 128, 256)
     int chain = 0;    // FP32 3D drift's y / z / y passes: 0 three passes; 1 / 2 one slab-ordered
                       // kernel over slabs of `chain` 8-column tiles (bit-identical, measured slower)
     int xstage = 0;   // FP32 x inverse + density + r2c pass (N >= 256): 1 = each warp copies its
