@@ -379,8 +379,14 @@ void Field::drift_update() {  // src/field.cxx:378-386
 
 
 // ---------------------------------------------------------------------------
-// autotuner cache: "v3 dim N dtype batch : x_rows y_tx la_tx tma nbuf pw plan wp ms"
+// autotuner cache: "v3 dim N dtype batch : x_rows y_tx la_tx tma nbuf pw plan wp ms : passes"
 // ---------------------------------------------------------------------------
+
+// Generation of the passes that a choice was timed among, at the end of its line.
+// A line of another generation, or of none (written before the plane-resident and
+// the FP64 warp-per-pencil passes), is not used: its plan or wp would switch
+// faster passes off.
+constexpr int kTunePasses = 2;
 
 static std::map<std::string, std::pair<Tune, double>>& tune_cache() {
     static std::map<std::string, std::pair<Tune, double>> c;
@@ -401,7 +407,11 @@ static bool tune_lookup(const std::string& key, const char* path, Tune& t, doubl
             std::istringstream vs(line.substr(colon + 3));
             Tune u;
             double m = 0.0;
-            if (vs >> u.x_rows >> u.y_tx >> u.la_tx >> u.tma >> u.nbuf >> u.pw >> u.plan >> u.wp >> m) c[key] = {u, m};
+            std::string sep;
+            int passes = 0;
+            if (vs >> u.x_rows >> u.y_tx >> u.la_tx >> u.tma >> u.nbuf >> u.pw >> u.plan >> u.wp >> m >> sep >> passes &&
+                sep == ":" && passes == kTunePasses)
+                c[key] = {u, m};
         }
         it = c.find(key);
     }
@@ -416,7 +426,7 @@ static void tune_store(const std::string& key, const char* path, const Tune& t, 
     if (path && *path) {
         std::ofstream out(path, std::ios::app);
         out << key << " : " << t.x_rows << " " << t.y_tx << " " << t.la_tx << " " << t.tma << " " << t.nbuf << " "
-            << t.pw << " " << t.plan << " " << t.wp << " " << ms << "\n";
+            << t.pw << " " << t.plan << " " << t.wp << " " << ms << " : " << kTunePasses << "\n";
     }
 }
 
