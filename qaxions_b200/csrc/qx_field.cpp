@@ -1416,6 +1416,14 @@ class FieldT final : public Field {
         // candidates: radix plan of the strided passes, pencils per thread, ring
         // depth, y / last-axis tile widths, rows per x block (plan 1 runs 8-column tiles)
         std::vector<Tune> cands;
+        // the direct-load and plane-resident passes, which take no geometry (x_rows: the
+        // row passes beside the direct-load ones)
+        if (Plane<R>::col(g_.N, g_.dim) || (g_.dim == 3 && Plane<R>::ycol(g_.N, g_.N / 2, -1)))
+            for (int xr : {0, 4}) {
+                Tune t;
+                t.x_rows = xr;
+                cands.push_back(t);
+            }
         const int pws[2] = {sizeof(R) == 4 ? 2 : 1, 1};
         const int nplans = Ops<R>::has_plan1(g_.N) ? 2 : 1;
         for (int plan = 0; plan < nplans; ++plan)
@@ -1465,8 +1473,12 @@ class FieldT final : public Field {
             tune_ = t;
             invalidate_graph();
             try {
-                time_steps(1, 1);  // warm-up, capture
-                const double ms = time_steps(nsteps, 1) / nsteps;
+                time_steps(1, 1);  // warm-up
+                // steps short enough for launches to count are timed as long calls run
+                // them, from graph replays (the first one uploads the graph)
+                const int n = time_steps(1, 1) < 1.0f ? std::max(nsteps, kGraphBodies + 1) : nsteps;
+                if (n > kGraphBodies) time_steps(n, 1);
+                const double ms = time_steps(n, 1) / n;
                 if (ms < best) {
                     best = ms;
                     best_t = t;
