@@ -2,9 +2,12 @@
 // qx_ops_f64.cu).
 #pragma once
 
+#include <map>
+#include <mutex>
 #include <stdexcept>
 #include <string>
 #include <type_traits>
+#include <utility>
 
 #include <cudaTypedefs.h>
 
@@ -69,6 +72,20 @@ static int x_rows_per_block(int N, long rows, int want) {
     return 1;
 }
 
+// Blocks of a row kernel that fit an SM at once, asked of the runtime once per
+// kernel and block: the same kernel runs with 1 to 8 rows per block, by the grid.
+static int x_blocks_per_sm(const void* kernel, int threads, size_t smem) {
+    static std::mutex lock;
+    static std::map<std::pair<const void*, int>, int> known;
+    std::lock_guard<std::mutex> hold(lock);
+    int& bps = known[{kernel, threads}];
+    if (!bps && (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kernel, threads, smem) != cudaSuccess || bps < 1)) {
+        cudaGetLastError();
+        bps = 1;
+    }
+    return bps;
+}
+
 template <typename R, int NN, typename K, typename... A>
 static long launch_x(K kernel, const XArgs<R>& x, int P, cudaStream_t st, int stage_elems = 0, A... args) {
     using C = cx_t<R>;
@@ -79,20 +96,7 @@ static long launch_x(K kernel, const XArgs<R>& x, int P, cudaStream_t st, int st
     set_smem(kernel, smem);
     // persistent grid: as many blocks as fit on the device at once (the
     // twiddle tables are staged once per block), at most one per P rows
-    static const void* cache_k[32] = {nullptr};
-    static int cache_bps[32] = {0};
-    int bps = 0;
-    for (int i = 0; i < 32 && cache_k[i]; ++i)
-        if (cache_k[i] == (const void*)kernel) bps = cache_bps[i];
-    if (!bps) {
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, kernel, T * P, smem) != cudaSuccess || bps < 1) bps = 1;
-        for (int i = 0; i < 32; ++i)
-            if (!cache_k[i]) {
-                cache_k[i] = (const void*)kernel;
-                cache_bps[i] = bps;
-                break;
-            }
-    }
+    const long bps = x_blocks_per_sm((const void*)kernel, T * P, smem);
     const long blocks = x.rows / P;
     long grid = (long)sm_count() * bps;
     if (grid > blocks) grid = blocks;
