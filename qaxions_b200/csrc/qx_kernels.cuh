@@ -785,9 +785,15 @@ template <> __device__ __forceinline__ float pois_mult<float>(long M2, const SAr
     return M2 == 0 ? (float)s.pois_g0 : (float)s.pois_c * __frcp_rn((float)M2);
 }
 // pois_c / M2 in FP64 without the general division's range checks: |n|^2 is an
-// integer below 2^24, exact in FP32, so its FP32 reciprocal takes two
-// Newton-Raphson steps to full precision, and the quotient one residual
-// correction (Markstein's division scheme), which rounds it as the division does
+// integer m below 2^24, exact in FP32, so its FP32 reciprocal takes two
+// Newton-Raphson steps to about full precision, and the quotient one residual
+// correction (Markstein's division scheme).  The result is the division's, away
+// from overflow and underflow: q is within a few units of its last place u of c / m,
+// so the residual c - q m, a multiple of u below 2^28 u, is exact, and its product
+// with x is within 2^-49 u of the missing part.  c / m is never that close to a
+// rounding boundary: with c = C 2^k u in 53-bit integers C, |C 2^k / m - (Q + 1/2)| =
+// |C 2^(k+1) - (2Q + 1) m| / 2m, an integer over 2m that is not 0 (2Q + 1 is odd and has
+// 54 bits, C has 53), so at least 2^-25.
 template <> __device__ __forceinline__ double pois_mult<double>(long M2, const SArgs<double>& s) {
     if (M2 == 0) return s.pois_g0;
     const double m = (double)(int)M2;
