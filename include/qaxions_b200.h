@@ -179,7 +179,8 @@ int qx_profile_step(qx_field_t *h, int nsteps, int max_entries, char *names, dou
  * plane-resident or direct-load passes (3D N = 32 ... 128, 2D N = 64 ... 512, FP32
  * 256^3) run them while every override that describes another form is 0: ring
  * depth, pencils per thread, tile columns of the pass, and x-pass rows for the
- * plane-resident ones. */
+ * plane-resident ones.  The kinetic sum of qx_mass_energy (one unstored transform per
+ * axis) has TMA-fed passes only, whatever tma is. */
 int qx_set_tune(qx_field_t *h, int x_rows, int y_tx, int la_tx, int tma, int nbuf, int pw);
 /* Radix plan of the TMA strided (y / last-axis) passes, no counterpart in the
  * reference (FFTW plans its own): 0 default, 1 the same radices in reverse

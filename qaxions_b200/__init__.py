@@ -427,7 +427,8 @@ class Field:
         persistent or the direct-load strided kernels (-1 keeps the current);
         pw: pencils per thread of the TMA passes (0 default, 1 or 2).  Grids
         with plane-resident or direct-load passes run them while no override
-        asks for the ring or the row blocks."""
+        asks for the ring or the row blocks; mass_energy's kinetic sum always
+        runs on the TMA-fed passes."""
         self._c("qx_set_tune", x_rows, y_tx, la_tx, tma, nbuf, pw)
 
     def set_plan(self, plan: int):

@@ -68,9 +68,10 @@ template <typename R> struct Ops {
     // last-axis pass
     static void la_pass(int N, const SP& s, int op, const Tune& tu, cudaStream_t st);
     // Diagnostics of psi (a.in, s.a) and V (a.Vin), one read of psi per axis
-    // (k_x_energy): per-block partials in part (7 * energy_blocks() doubles):
-    // five arrays of n[0] from the x rows back to back, then at 5 and 6 *
-    // energy_blocks() the n[1] y and n[2] z shares of sum n^2 |F_axis psi|^2
+    // (k_x_energy; the y and z shares on the TMA-fed passes for either tu.tma):
+    // per-block partials in part (7 * energy_blocks() doubles): five arrays of n[0]
+    // from the x rows back to back, then at 5 and 6 * energy_blocks() the n[1] y and
+    // n[2] z shares of sum n^2 |F_axis psi|^2
     static void energy(int N, const XP& a, const SP& s, double* part, long (&n)[3], const Tune& tu, cudaStream_t st);
     static long energy_blocks();
     // The drift chain (y forward, z forward + drift + z inverse, y inverse) of a
