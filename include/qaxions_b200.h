@@ -258,9 +258,9 @@ int qx_sync(qx_field_t *h);
  * runs one box per process, src/main.cxx:34-53) ----
  * ngroups groups of boxes; group g holds boxes[g] boxes of size N[g]^dim, all
  * with the same L, pref, dtype and dt.  The boxes of a group are stacked in one
- * device array, so every pass of a step is one persistent launch over the
- * tiles of all of the group's boxes; each group's loop body is replayed from a
- * CUDA graph on its own stream and the groups run concurrently.  Boxes are
+ * device array, so every pass of a step is one launch over the planes or tiles
+ * of all of the group's boxes; the groups' loop bodies are branches of one CUDA
+ * graph of several steps and run concurrently.  Boxes are
  * numbered group by group.  Single-box operations (spectrum, Vhat, FFT plugin)
  * are not available on ensemble boxes.  Errors: qx_ens_last_error(h). */
 typedef struct qx_ens_s qx_ens_t;
@@ -288,8 +288,8 @@ int qx_ens_time_steps(qx_ens_t *h, int nsteps, float *ms);
 /* mass sum |psi|^2 dV of every box (nboxes doubles) */
 int qx_ens_mass(qx_ens_t *h, double *M);
 /* Loop-body mode of the steps in between the first and the last of a call.
- * mixed = 0 (default): each group's body replayed on its own stream (a graph
- * branch per group, one launch per pass per group).  mixed = 1: the whole
+ * mixed = 0 (default): each group's bodies in a graph branch of their own, one
+ * launch per pass per group.  mixed = 1: the whole
  * loop body of every box as ONE persistent launch per step, driven by a work
  * queue of (pass, box, tile-or-rows) units (pass by pass, the costliest sizes
  * first); a unit starts once its box has finished the previous pass, so the

@@ -521,8 +521,9 @@ class Ensemble:
 
     ``groups`` is a list of (N, count): count boxes of N^dim sites each.  Boxes
     of one size share one batched device array, so each pass of a step is one
-    persistent launch over all of their tiles; groups run concurrently, each
-    replaying its loop body from a CUDA graph.  With ``mixed=True`` (3D, at
+    launch over all of their planes or tiles; groups run concurrently, as
+    branches of one CUDA graph of eight steps (short calls launch their passes
+    one by one).  With ``mixed=True`` (3D, at
     most 4 sizes from 16, 32, 64, 96, 128) the loop body of every box is
     instead ONE persistent launch per step, fed by a work queue of (pass, box,
     tile) units in which a unit starts once its box has finished the previous

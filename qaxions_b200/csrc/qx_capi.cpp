@@ -465,8 +465,9 @@ struct qx_ens_s {
     std::vector<int> index_in;  // box -> index within its group
     long long sites = 0;
     std::string err;
-    // one loop body of every group as ONE graph (a branch per group on the
-    // group's stream, forked from and joined into `s0`), replayed once per step
+    // loop bodies of every group as ONE graph (a branch per group on the group's
+    // stream, forked from and joined into `s0`): kEnsGraphBodies steps per replay, one
+    // in the mixed-size modes
     cudaStream_t s0 = nullptr;
     cudaGraphExec_t exec = nullptr;
     std::vector<double> exec_dt;  // each group's ds when captured

@@ -153,7 +153,7 @@ class Field {
     void drift_update();
     virtual void propagate() = 0;
     // merged leapfrog of src/main.cxx:64-85 (measurements off), fused passes,
-    // loop body replayed from a CUDA graph
+    // loop bodies replayed from a CUDA graph where a call has enough of them
     virtual void step(int nsteps) = 0;
     // step() in pieces, for a caller that replays several fields' loop bodies
     // in one CUDA graph of its own (an ensemble; STATIC cosmology): the

@@ -11,7 +11,7 @@
 //   k_plane_inv         y inverse, x inverse -> psi; density, x r2c, y -> rho^
 //   k_col<OP_POISSON>   rho^: z forward, -1/k^2, z inverse (column 0 included)
 //   k_plane_c2r         y inverse, x c2r -> V; kick, x forward, y -> psi^_xy
-// and L2 sees 16w + 8w bytes per site (w = bytes per real) instead of 28w.
+// and L2 sees 16w bytes per site (w = bytes per real: 4w, 5w, 2w, 5w) instead of 28w.
 // Between the launches psi is transformed along x and y (psi^_xy).
 // Measured (one B200, us per step, nine launches -> these four): 32^3 FP32 45.7
 // -> 18.6, 64^3 FP32 45.7 -> 33.0, 128^3 FP32 91 -> 60, 96^3 FP64 99 -> 73.
@@ -21,7 +21,8 @@
 // accesses are free of bank conflicts and a warp's twiddle loads are
 // broadcasts.  Row phases (x): a row's threads sit in one warp, as in the row
 // passes.  The butterflies, twiddles and their order are those of the row and
-// pencil passes, so the results agree with theirs bit for bit in FP32.
+// pencil passes: psi agrees with theirs bit for bit in FP32, V to 5e-8 (the compiler
+// fuses the Poisson scale with the next addition in another order).
 //
 // Every kernel stages its tables, then waits for the kernel before it
 // (griddepcontrol.wait) before it touches the state: launched with programmatic
