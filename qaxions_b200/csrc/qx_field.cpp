@@ -57,18 +57,21 @@ struct DevBuf {
     template <typename T> T* as() const { return static_cast<T*>(p); }
 };
 
-// Pins one line of host memory, once, for as long as the process runs.  The driver
-// pins in large blocks and gives a block back with the last allocation in it: the
-// first small cudaHostAlloc of a process takes 1.5 to 2.5 ms and the last cudaFreeHost
-// 0.4 ms, those in between 2 and 3 us.  With this line held every field's ResultBuf
-// is one in between (construction of a 3D 32^3 FP32 field 3.1 -> 0.6 ms).
+// Pins one line of host memory per device, for as long as the process runs.  The
+// driver pins in large blocks and gives a block back with the last allocation in it:
+// the first small cudaHostAlloc takes 1.5 to 2.5 ms and the last cudaFreeHost 0.4 ms,
+// those in between 2 and 3 us.  With this line held every field's ResultBuf is one in
+// between (construction of a 3D 32^3 FP32 field 3.1 -> 0.6 ms).
 static void hold_pinned_block() {
-    static std::atomic<bool> held{false};
-    if (held.exchange(true)) return;
+    static std::atomic<unsigned long long> held{0};
+    int dev = 0;
+    QX_CUDA(cudaGetDevice(&dev));
+    const unsigned long long bit = 1ull << (dev & 63);
+    if (held.fetch_or(bit) & bit) return;
     void* p = nullptr;
     if (cudaHostAlloc(&p, 64, cudaHostAllocMapped) != cudaSuccess) {
         cudaGetLastError();  // fields pin their own, at the price above
-        held = false;
+        held &= ~bit;
     }
 }
 
