@@ -224,7 +224,7 @@ int qx_set_chain(qx_field_t *h, int on);
 /* Autotuner: time nsteps steps under each candidate launch geometry (radix
  * plan of the strided passes, pencils per thread, TMA ring depth, tile widths,
  * rows per x block, and the plane-resident and direct-load passes, which take no
- * geometry), keep the fastest; psi is restored afterwards.  Steps below a
+ * geometry), keep the fastest; psi, clock and cosmology are restored afterwards.  Steps below a
  * millisecond are timed from graph replays, at least 9 of them.  Cached per
  * (dim, N, dtype, batch) in the process and in the text file cache_path if not
  * NULL (read first, appended after); fields created later with the same key

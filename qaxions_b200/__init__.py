@@ -488,8 +488,8 @@ class Field:
         self._c("qx_set_clock", step, time)
 
     def autotune(self, nsteps: int = 3, cache: str | None = None):
-        """Pick the fastest launch geometry for this grid (psi is left as it
-        was).  Returns (ms per step of the choice, whether it came from the
+        """Pick the fastest launch geometry for this grid (psi, clock and
+        cosmology are left as they were).  Returns (ms per step of the choice, whether it came from the
         cache); `cache` names a text file shared between runs."""
         ms = C.c_double()
         fc = C.c_int()
